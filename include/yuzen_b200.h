@@ -105,7 +105,9 @@ int yz_solver_set_amg_reuse(yz_solver* s, int max_solves);
 /* The BiCGStab loop as one CUDA graph launch per solve (1, the default) or
  * launched from the stream with one iteration in flight (0).  The graph is
  * captured from the context's stream in thread-local capture mode, so other
- * host threads may drive their own contexts (and allocate) meanwhile. */
+ * host threads may drive their own contexts (and allocate) meanwhile.  The
+ * loop of a small system (FP64: up to 20,000 rows) is one launch of a
+ * thread-block cluster either way. */
 int yz_solver_set_graph_loop(yz_solver* s, int on);
 
 /* ILinearSolverBackend::Memory / SetMemory (LinearSolverBackend.h:89-102):

@@ -421,3 +421,13 @@ def test_tuning_shapes_and_sweeps():
         assert g[0] == 0 and g[2] <= float(d["epsilon"]), (shape, g[:3])
         its[shape] = g[1]
     assert its[(-1, 0, 0)] < its[(-1, 0, 1)], its
+
+
+@pytest.mark.parametrize("N,periodic", [(51, False), (52, True), (60, False), (61, True), (124, False), (137, True),
+                                        (138, False)])
+def test_cluster_run_bitwise(N, periodic):
+    """The run in one cluster (yz_cluster.cuh) from the smallest systems with
+    a coarse level to the largest it takes (20,000 rows) and the first beyond
+    it, with the last chunk of 256 rows full (60, 124) and not."""
+    d = _systems.film_system(N, seed=N, periodic=periodic)
+    assert_same(gpu_solve(d)[:4], _oracle.OracleSolver().solve(d))

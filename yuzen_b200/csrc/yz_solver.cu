@@ -9,6 +9,7 @@
 // a breakdown answered by the residual check of :681-713.
 #include "yz_amg_kernels.cuh"
 #include "yz_coarse.cuh"
+#include "yz_cluster.cuh"
 #include "yz_learned.h"
 #include "yz_solver_impl.h"
 #include "yz_prof.h"
@@ -688,9 +689,12 @@ void Solver::Cycle(size_t l, const double *f, double *x)
 		Level &C = *_levels[l + 1];
 		YZ_LAUNCH(KPreSmoothResidual, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
 		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, x, L.t.get());
-		YZ_LAUNCH(KRestrict, GridFor((long long)C.n * 4, kB), kB, 0, _st, Halt(), C.n, L.rptr.get(), L.rcol.get(),
-		          L.rval.get(), L.t.get(), C.f.get());
-		Cycle(l + 1, C.f.get(), C.x.get());
+		if(l > 0 || !LaunchCoarse<double>())
+		{
+			YZ_LAUNCH(KRestrict, GridFor((long long)C.n * 4, kB), kB, 0, _st, Halt(), C.n, L.rptr.get(), L.rcol.get(),
+			          L.rval.get(), L.t.get(), C.f.get());
+			Cycle(l + 1, C.f.get(), C.x.get());
+		}
 		YZ_LAUNCH(KProlong, g, kB, 0, _st, Halt(), n, L.pptr.get(), L.pcol.get(), L.pval.get(), C.x.get(), x, L.xt.get());
 		YZ_LAUNCH(KPostSmooth, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
 		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x);
@@ -754,9 +758,12 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 		if(la == 1)
 			YZ_LAUNCH_PDL((KPreSmoothResidual<float, TF, float>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
 			          val, L.M32.get(), f, L.x32.get(), L.t32.get());
-		YZ_LAUNCH_PDL(KRestrict<float>, GridFor((long long)C.n * 4, kB), kB, 0, _st, Halt(), C.n, L.rptr.get(), L.rcol.get(),
-		          L.rval32.get(), L.t32.get(), C.f32.get());
-		Cycle32<float, float>(l + 1, C.f32.get(), C.x32.get());
+		if(l > 0 || !LaunchCoarse<float>())
+		{
+			YZ_LAUNCH_PDL(KRestrict<float>, GridFor((long long)C.n * 4, kB), kB, 0, _st, Halt(), C.n, L.rptr.get(), L.rcol.get(),
+			              L.rval32.get(), L.t32.get(), C.f32.get());
+			Cycle32<float, float>(l + 1, C.f32.get(), C.x32.get());
+		}
 		if(lp > 1)
 			CoarseProlong(lp, n, L.pptr.get(), L.pcol.get(), L.pval32.get(), C.x32.get(), L.x32.get(), L.xt32.get());
 		else
@@ -1032,6 +1039,148 @@ void Solver::SetLearned(Learned *L, int mode, int collectSolves, int perSolve, d
 	_offLearned = TryBackoff();
 }
 
+//--------------------------------------------------------------------------
+//  one cluster (yz_cluster.cuh)
+//--------------------------------------------------------------------------
+namespace {
+template<class T> void FillLevel(ClLevel<T> &c, const Level &L, bool last)
+{
+	c.n = L.n;
+	c.direct = L.direct ? 1 : 0;
+	c.last = (!L.direct && last) ? 1 : 0;
+	c.ptr = L.ptr.get(); c.col = L.col.get();
+	c.rptr = L.rptr.get(); c.rcol = L.rcol.get();
+	c.pptr = L.pptr.get(); c.pcol = L.pcol.get();
+	if constexpr(std::is_same<T, double>::value)
+	{
+		c.val = L.val.get(); c.M = L.M.get(); c.inv = L.inv.get(); c.rval = L.rval.get(); c.pval = L.pval.get();
+		c.f = L.f.get(); c.x = L.x.get(); c.t = L.t.get(); c.xt = L.xt.get();
+	}
+	else
+	{
+		c.val = L.val32.get(); c.M = L.M32.get(); c.inv = L.inv32.get(); c.rval = L.rval32.get(); c.pval = L.pval32.get();
+		c.f = L.f32.get(); c.x = L.x32.get(); c.t = L.t32.get(); c.xt = L.xt32.get();
+	}
+}
+
+template<class K, class... A> void LaunchCluster(K kernel, int size, cudaStream_t st, const char *name, A... args)
+{
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3(size);
+	cfg.blockDim = dim3(kClT);
+	cfg.stream = st;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeClusterDimension;
+	attr[0].val.clusterDim.x = size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	const bool timed = TimedKernel(name);
+	if(timed) TimeBegin(st);
+	Check(cudaLaunchKernelEx(&cfg, kernel, args...), name);
+	if(timed) TimeEnd(st);
+	CountLaunches(1);
+}
+
+//  16 blocks (beyond the portable 8) where the device takes such a cluster; a
+//  fact of the device, asked once for each (the question takes milliseconds)
+template<auto kernel> int ClusterBlocks(int device)
+{
+	static std::mutex m;
+	static std::map<int, int> known;
+	std::lock_guard<std::mutex> lk(m);
+	const auto it = known.find(device);
+	if(it != known.end()) return it->second;
+	int &blocks = known[device];
+	blocks = 0;
+	YZ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+	for(int size = 16; size >= 8; size /= 2)
+	{
+		cudaLaunchConfig_t cfg = {};
+		cfg.gridDim = dim3(size);
+		cfg.blockDim = dim3(kClT);
+		cudaLaunchAttribute attr[1];
+		attr[0].id = cudaLaunchAttributeClusterDimension;
+		attr[0].val.clusterDim.x = size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+		cfg.attrs = attr;
+		cfg.numAttrs = 1;
+		int count = 0;
+		if(cudaOccupancyMaxActiveClusters(&count, kernel, &cfg) == cudaSuccess && count > 0) return blocks = size;
+		(void)cudaGetLastError();
+	}
+	return 0;
+}
+} // namespace
+
+template<class T> bool Solver::FillPlan(ClPlan<T> &P) const
+{
+	if(_nlev > (size_t)kClMaxLevels) return false;
+	P.count = (int)_nlev;
+	P.sweeps = std::is_same<T, float>::value ? FineSweeps() : 1;
+	P.so = _sellOff.get();
+	P.sn = _sten;
+	for(size_t l = 0; l < _nlev; ++l) FillLevel(P.lv[l], *_levels[l], l + 1 == _nlev);
+	P.lv[0].col = _sellCol.get();
+	if constexpr(std::is_same<T, double>::value) P.lv[0].val = _sellVal.get();
+	else P.lv[0].val = _sellVal32.get();
+	return true;
+}
+
+//  The run as one launch of a cluster; false: it does not fit one
+template<class V, class T> bool Solver::LaunchLoop(int kind, const V *val)
+{
+	static_assert(sizeof(ClPlan<T>) + sizeof(ClSystem<V>) < 4000, "kernel parameters");
+	const int size = ClusterBlocks<KLoopCluster<V, T>>(_device);
+	if(!size) return false;
+	ClPlan<T> P = {};
+	if(kind == kPrecAmg && !FillPlan(P)) return false;
+	ClSystem<V> S;
+	S.n = _n;
+	S.ptr = _levels[0]->ptr.get(); S.so = _sellOff.get(); S.col = _sellCol.get();
+	S.sn = _sten;
+	S.val = val;
+	S.m = kind == kPrecDiag ? _m.get() : nullptr;
+	S.x = _x.get(); S.r = _r.get(); S.rh = _rh.get(); S.p = _p.get(); S.v = _v.get(); S.s = _s.get();
+	S.ph = _ph.get(); S.sh = _sh.get(); S.t = _t.get();
+	S.sc = _sc.get();
+	LaunchCluster(KLoopCluster<V, T>, size, _st, "KLoopCluster", S, P);
+	return true;
+}
+
+bool Solver::ClusterRun(int kind)
+{
+	if(kind == kPrecLearned || _n > ClusterRows()) return false;
+	if(_precision == YZ_PREC_FP32_MATRIX) return LaunchLoop<float, float>(kind, _sellVal32.get());
+	if(_precision == YZ_PREC_FP32_CYCLE) return LaunchLoop<double, float>(kind, _sellVal.get());
+	return LaunchLoop<double, double>(kind, _sellVal.get());
+}
+
+//  The largest system whose run is one cluster's (YZ_CLUSTER_ROWS sets it).
+//  Sixteen multiprocessors lose to the whole chip once a phase is bound by
+//  its rows: FP64 steps of three solves (iterations, ms, separate launches
+//  against one cluster) 5.2 / 2.9 at 4,624 rows, 5.1 / 3.8 at 10,000, 4.8 /
+//  4.4 at 17,424, 4.8 / 5.3 at 26,896; the FP32 cycle with its extra sweeps
+//  1.6 / 1.0, 1.6 / 1.3, 1.65 / 1.75, 1.8 / 2.3.
+int Solver::ClusterRows() const
+{
+	static const char *env = std::getenv("YZ_CLUSTER_ROWS");
+	static const int set = env ? std::min(std::atoi(env), kClMaxChunks * kRChunk) : -1;
+	if(set >= 0) return set;
+	return _precision == YZ_PREC_FP64 ? 20000 : 14000;
+}
+
+//  the levels below the finest in one launch of a cluster
+template<class T> bool Solver::LaunchCoarse()
+{
+	static const char *env = std::getenv("YZ_CLUSTER_COARSE");
+	if(env && env[0] == '0') return false;
+	ClPlan<T> P = {};
+	if(_nlev < 2 || !FillPlan(P)) return false;
+	const int size = ClusterBlocks<KCoarseCluster<T>>(_device);
+	if(!size) return false;
+	LaunchCluster(KCoarseCluster<T>, size, _st, "KCoarseCluster", Halt(), P);
+	return true;
+}
+
 void Solver::ApplyPrec(int kind, const double *r, double *z)
 {
 	const int n = _n;
@@ -1101,7 +1250,7 @@ void Solver::RunIterations(int kind)
 		++hooks;
 	};
 	if(collect) _zs.reserve((size_t)_n);
-	if(graphOff || !_graphLoop || TimingActive() || collect)
+	if(graphOff || TimingActive() || collect || (!_graphLoop && (kind == kPrecLearned || _n > ClusterRows())))
 	{
 		//  one iteration kept in flight: the state after iteration k is
 		//  copied to pinned memory and read while iteration k+1 runs; the
@@ -1144,13 +1293,17 @@ void Solver::RunIterations(int kind)
 		if(collect) { --_collectLeft; _collected += hooks; }
 		return;
 	}
-	if(lg.exec == nullptr || lg.key != key)
+	const bool cluster = ClusterRun(kind);
+	if(!cluster)
 	{
-		FreeLoopGraph(lg);
-		BuildLoopGraph(kind, lg);
-		lg.key = key;
+		if(lg.exec == nullptr || lg.key != key)
+		{
+			FreeLoopGraph(lg);
+			BuildLoopGraph(kind, lg);
+			lg.key = key;
+		}
+		YZ_CUDA(cudaGraphLaunch(lg.exec, _st));
 	}
-	YZ_CUDA(cudaGraphLaunch(lg.exec, _st));
 	//  the end of the run queued behind the loop -- its time, the answer
 	//  into the caller's x (Solve's tail) -- so that one wait covers all
 	YZ_CUDA(cudaEventRecord(_ev2, _st));
@@ -1161,7 +1314,7 @@ void Solver::RunIterations(int kind)
 	}
 	ReadScal();
 	//  the kernels the loop ran
-	CountLaunches(lg.perBody * (long long)_hsc->bodies);
+	if(!cluster) CountLaunches(lg.perBody * (long long)_hsc->bodies);
 }
 
 void Solver::FreeLoopGraph(LoopGraph &g)

@@ -10,6 +10,7 @@
 namespace yz {
 
 class Learned;
+template<class T> struct ClPlan;
 
 //  Scalars of one BiCGStab run, in device memory (written by the block that
 //  folds a reduction, read by the element-wise kernels and by the host).
@@ -102,6 +103,12 @@ private:
 	void RoundCycle();
 	template<class TF, class TX> void Cycle32(size_t l, const TF *f, TX *x);
 	int LanesFor(long long nnz, int n) const;
+	//  the runs and coarse levels that one cluster takes (yz_cluster.cuh)
+	template<class T> bool FillPlan(ClPlan<T> &P) const;
+	template<class V, class T> bool LaunchLoop(int kind, const V *val);
+	template<class T> bool LaunchCoarse();
+	bool ClusterRun(int kind);
+	int ClusterRows() const;
 	bool CoarseCycleOn() const;
 	static int CoarseBlocksPerSm();
 	void LaunchCoarseCycle();
