@@ -431,3 +431,32 @@ def test_cluster_run_bitwise(N, periodic):
     it, with the last chunk of 256 rows full (60, 124) and not."""
     d = _systems.film_system(N, seed=N, periodic=periodic)
     assert_same(gpu_solve(d)[:4], _oracle.OracleSolver().solve(d))
+
+
+def _swapping_system(n: int, seed: int) -> dict:
+    """n rows whose largest entries lie off the diagonal (a shift by a third
+    of n), with a band and scattered entries around them: the direct level's
+    elimination swaps rows in nearly every step."""
+    rng = np.random.default_rng(seed)
+    cols = [{i, (i + n // 3) % n} | {(i + o) % n for o in (-2, -1, 1, 2)} |
+            set(rng.integers(0, n, 3).tolist()) for i in range(n)]
+    rows = [[i] + sorted(c - {i}) for i, c in enumerate(cols)]
+    rowptr = np.zeros(n + 1, np.int32)
+    rowptr[1:] = np.cumsum([len(r) for r in rows])
+    col = np.array([c for r in rows for c in r], np.int32)
+    own = np.repeat(np.arange(n), np.diff(rowptr))
+    val = rng.standard_normal(col.size)
+    val[col == (own + n // 3) % n] += 9.0
+    scol, ssrc = _systems.sorted_mirror(rowptr, col)
+    return {"n": n, "nnz": col.size, "rowptr": rowptr, "col": col, "sorted_col": scol, "sorted_src": ssrc,
+            "values": val, "rhs": rng.standard_normal(n), "x0": np.zeros(n), "precondition": 2, "scaling": 0,
+            "max_iteration": 20, "epsilon": 1e-13, "conc": 0}
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 17, 31, 33, 65, 255, 257, 511, 513, 1023, 1025, 1100])
+def test_direct_level_bitwise(n):
+    """The direct level's inverse (yz_gj.cuh) around its widths: a column
+    tile (16), a panel (32 slots, fewer above ~810 rows), the rows a block
+    takes side by side (256, 512, 1024)."""
+    d = _swapping_system(n, n)
+    assert_same(gpu_solve(d)[:4], _oracle.OracleSolver().solve(d))

@@ -624,170 +624,6 @@ __global__ void KGemmCompact(int nx, const int *__restrict__ cptr, const int *__
 }
 
 //--------------------------------------------------------------------------
-//  Gauss-Jordan inverse of the coarsest level on [A | I] with partial
-//  pivoting (the oracle's GaussJordanInverse, yzo_solver.cpp), blocked.
-//  Step k of the unblocked algorithm changes every column j >= k by the same
-//  rule, in which only the column's own values, the pivot row p_k, the pivot
-//  piv_k and the multipliers f_k(i) = M[src_i][k] (column k before the step,
-//  src_i = k for i = p_k, else i) appear:
-//      row k:    M[k][j] = M[p][j] / piv
-//      row i:    M[i][j] = f == 0 ? M[src_i][j] : M[src_i][j] - f M[k][j]
-//  so a panel of B consecutive columns is run through its B steps by one
-//  block (recording p, piv and f of each), and every later column then
-//  replays those B steps on its own.  Each element sees exactly the
-//  operations of the unblocked algorithm, in the same order: the result is
-//  the oracle's to the bit, in 2 n / B launches instead of n.
-//  M is held column-major (column j at Mc + j n), n <= 3000.
-//--------------------------------------------------------------------------
-__global__ void KGjInit(int n, const int *__restrict__ ptr, const int *__restrict__ col,
-                        const double *__restrict__ val, double *__restrict__ Mc)
-{
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-	{
-		for(int k = ptr[i]; k < ptr[i + 1]; ++k) Mc[(size_t)col[k] * n + i] = val[k];
-		Mc[(size_t)(n + i) * n + i] = 1.0;
-	}
-}
-
-__device__ __forceinline__ void GjBetter(double &best, int &idx, double a, int ia)
-{
-	if(a > best || (a == best && ia < idx)) { best = a; idx = ia; }
-}
-
-//  the pivot of column c of the panel among rows k..n-1: the first row of
-//  the largest |a|, taken only when larger than |a_kk| (the sequential
-//  rule); the largest |a| (first row among equals) over each warp by
-//  shuffles, then over the warps' results -- the same choice as any order of
-//  comparison (a NaN is never taken, as in the sequential scan)
-__device__ __forceinline__ int GjPivot(const double *colc, int n, int k, double *rv, int *ri)
-{
-	const int t = threadIdx.x, nt = blockDim.x, lane = t & 31, w = t >> 5;
-	double best = -1.0; int idx = n;
-	for(int i = k + t; i < n; i += nt) GjBetter(best, idx, fabs(colc[i]), i);
-	for(int off = 16; off >= 1; off >>= 1)
-	{
-		const double a = __shfl_down_sync(0xffffffffu, best, off);
-		const int ia = __shfl_down_sync(0xffffffffu, idx, off);
-		GjBetter(best, idx, a, ia);
-	}
-	if(lane == 0) { rv[w] = best; ri[w] = idx; }
-	__syncthreads();
-	if(w == 0)
-	{
-		const int nw = nt >> 5;
-		best = (lane < nw) ? rv[lane] : -1.0; idx = (lane < nw) ? ri[lane] : n;
-		for(int off = 16; off >= 1; off >>= 1)
-		{
-			const double a = __shfl_down_sync(0xffffffffu, best, off);
-			const int ia = __shfl_down_sync(0xffffffffu, idx, off);
-			GjBetter(best, idx, a, ia);
-		}
-		if(lane == 0) { rv[32] = best; ri[32] = idx; }
-	}
-	__syncthreads();
-	const int p = (rv[32] > fabs(colc[k])) ? ri[32] : k;
-	__syncthreads();
-	return p;
-}
-
-//  one block of 512 threads: the B columns k0..k0+B-1, their steps; records
-//  pivRow, pivVal and F (B x n) for the columns after them
-__global__ void __launch_bounds__(512) KGjPanel(int n, int k0, int B, const double *__restrict__ Mc,
-                                                double *__restrict__ F, int *__restrict__ pivRow,
-                                                double *__restrict__ pivVal)
-{
-	extern __shared__ double smem[];
-	double *P = smem;                                  // B columns of n
-	double *rv = smem + (size_t)B * n;                 // 512 reduction values
-	int *ri = reinterpret_cast<int *>(rv + 512);       // 512 reduction indices
-	__shared__ double spiv;
-	const int t = threadIdx.x, nt = blockDim.x;
-	for(int e = t; e < B * n; e += nt) P[e] = Mc[(size_t)k0 * n + e];
-	__syncthreads();
-	const int lane = t & 31, warp = t >> 5, nw = nt >> 5;
-	for(int c = 0; c < B; ++c)
-	{
-		const int k = k0 + c;
-		double *colc = P + (size_t)c * n;
-		const int p = GjPivot(colc, n, k, rv, ri);
-		if(t == 0) { spiv = colc[p]; pivRow[c] = p; pivVal[c] = colc[p]; }
-		//  the multipliers, column c before the step
-		for(int i = t; i < n; i += nt) F[(size_t)c * n + i] = colc[(i == p) ? k : i];
-		__syncthreads();
-		const double piv = spiv;
-		//  the step on the panel's columns c..B-1, one warp per column
-		for(int cc = c + warp; cc < B; cc += nw)
-		{
-			double *cl = P + (size_t)cc * n;
-			const double colp = cl[p], colk = cl[k];
-			__syncwarp();
-			const double rowK = colp / piv;
-			for(int i = lane; i < n; i += 32)
-			{
-				double out;
-				if(i == k) out = rowK;
-				else
-				{
-					const int src = (i == p) ? k : i;
-					const double f = F[(size_t)c * n + i];
-					const double mij = (src == k) ? colk : cl[i];
-					out = (f == 0.0) ? mij : mij - f * rowK;
-				}
-				cl[i] = out;
-			}
-			__syncwarp();
-		}
-		__syncthreads();
-	}
-}
-
-//  every column j >= jStart replays the panel's B steps; one block per column
-__global__ void KGjUpdate(int n, int k0, int B, int jStart, double *__restrict__ Mc, const double *__restrict__ F,
-                          const int *__restrict__ pivRow, const double *__restrict__ pivVal)
-{
-	extern __shared__ double colv[];
-	__shared__ double sColp, sColk;
-	const int j = jStart + blockIdx.x;
-	const int t = threadIdx.x, nt = blockDim.x;
-	double *g = Mc + (size_t)j * n;
-	for(int i = t; i < n; i += nt) colv[i] = g[i];
-	__syncthreads();
-	for(int c = 0; c < B; ++c)
-	{
-		const int k = k0 + c, p = pivRow[c];
-		if(t == 0) { sColp = colv[p]; sColk = colv[k]; }
-		__syncthreads();
-		const double rowK = sColp / pivVal[c], colk = sColk;
-		for(int i = t; i < n; i += nt)
-		{
-			double out;
-			if(i == k) out = rowK;
-			else
-			{
-				const int src = (i == p) ? k : i;
-				const double f = F[(size_t)c * n + i];
-				const double mij = (src == k) ? colk : colv[i];
-				out = (f == 0.0) ? mij : mij - f * rowK;
-			}
-			colv[i] = out;
-		}
-		__syncthreads();
-	}
-	for(int i = t; i < n; i += nt) g[i] = colv[i];
-}
-
-//  the right half of [I | A^-1], row-major
-__global__ void KGjExtract(int n, const double *__restrict__ Mc, double *__restrict__ inv)
-{
-	const long long total = (long long)n * n;
-	for(long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x)
-	{
-		const int i = (int)(e / n), j = (int)(e % n);
-		inv[(size_t)i * n + j] = Mc[(size_t)(n + j) * n + i];
-	}
-}
-
-//--------------------------------------------------------------------------
 //  V-cycle.  Every kernel of the solve's iteration takes halt, the state
 //  word of its BiCGStab run (non-zero once it has stopped), and does nothing
 //  when it is set: the iterations are queued ahead of the host's check.

@@ -9,6 +9,7 @@
 // a breakdown answered by the residual check of :681-713.
 #include "yz_amg_kernels.cuh"
 #include "yz_coarse.cuh"
+#include "yz_gj.cuh"
 #include "yz_cluster.cuh"
 #include "yz_learned.h"
 #include "yz_solver_impl.h"
@@ -522,43 +523,34 @@ int Solver::Gemm(int nx, const int *xptr, const int *xcol, const double *xval, c
 	return nnz;
 }
 
-//  The dense inverse of the direct level (KGjPanel / KGjUpdate): panels of B
-//  columns, B as large as fits the panel block's shared memory (32 below
-//  ~770 rows)
+//  The dense inverse of the direct level (yz_gj.cuh): a launch a panel of
+//  slots, applying it and factoring the next
 void Solver::DirectInverse(Level &L)
 {
 	const int n = L.n;
 	if(n > 3000) throw UsageError("AMG set-up: the direct level has more than 3000 rows");
-	const size_t w = 2 * (size_t)n;
-	_gj[0].reserve((size_t)n * w);
-	_gj[1].reserve((size_t)32 * n);
-	_gjPiv.reserve(32);
-	_gjRow.reserve(32);
-	double *Mc = _gj[0].get(), *F = _gj[1].get();
-	YZ_CUDA(cudaMemsetAsync(Mc, 0, (size_t)n * w * sizeof(double), _st));
-	YZ_LAUNCH(KGjInit, GridFor(n, kB), kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), Mc);
-	const size_t maxSmem = 200 * 1024;
-	int B = (int)std::min<size_t>(32, (maxSmem - 512 * 12) / ((size_t)n * sizeof(double)));
-	if(B < 1) B = 1;
-	static bool attrSet = false;
-	if(!attrSet)
+	const int B = GjPanelWidth(n);
+	_gj[0].reserve((size_t)n * n);
+	_gj[1].reserve((size_t)2 * B * n);
+	_gjPan.reserve(2);
+	_gjOrig.reserve((size_t)n);
+	double *Mc = _gj[0].get(), *F[2] = {_gj[1].get(), _gj[1].get() + (size_t)B * n};
+	YZ_CUDA(cudaMemsetAsync(Mc, 0, (size_t)n * n * sizeof(double), _st));
+	YZ_LAUNCH(KGjInit, GridFor(n, kB), kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), Mc, _gjOrig.get());
+	auto kernel = n <= 256 ? KGjStep<16, 1, 2, 1> : n <= 512 ? KGjStep<16, 1, 1, 1> : n <= 1024 ? KGjStep<16, 2, 1, 1> :
+	              n <= 2048 ? KGjStep<8, 4, 1, 2> : KGjStep<8, 6, 1, 2>;
+	const int tiles = std::min((n + kGjCols - 1) / kGjCols, 147);
+	for(int q = -1, k = 0; q < 0 || k - B < n; ++q)
 	{
-		YZ_CUDA(cudaFuncSetAttribute(KGjPanel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)maxSmem));
-		YZ_CUDA(cudaFuncSetAttribute(KGjUpdate, cudaFuncAttributeMaxDynamicSharedMemorySize, 3000 * 8));
-		attrSet = true;
-	}
-	for(int k0 = 0; k0 < n; k0 += B)
-	{
-		const int b = std::min(B, n - k0);
-		const size_t smem = (size_t)b * n * sizeof(double) + 512 * (sizeof(double) + sizeof(int));
-		YZ_LAUNCH(KGjPanel, 1, 512, smem, _st, n, k0, b, Mc, F, _gjRow.get(), _gjPiv.get());
-		const int jStart = k0 + b, cols = (int)w - jStart;
-		if(cols > 0)
-			YZ_LAUNCH(KGjUpdate, cols, 128, (size_t)n * sizeof(double), _st, n, k0, b, jStart, Mc, F, _gjRow.get(),
-			          _gjPiv.get());
+		//  panel q (from k - B on) applied, the next one (from k on) factored
+		const GjPanel *prev = q < 0 ? nullptr : _gjPan.get() + (q & 1);
+		const int bNext = std::max(0, std::min(B, n - k));
+		YZ_LAUNCH(kernel, q < 0 ? 1 : 1 + tiles, kGjThreads, 0, _st, n, Mc, prev, F[q & 1], _gjPan.get() + ((q + 1) & 1),
+		          F[(q + 1) & 1], k, bNext, _gjOrig.get());
+		k += B;
 	}
 	L.inv.reserve((size_t)n * n);
-	YZ_LAUNCH(KGjExtract, GridFor((long long)n * n, kB), kB, 0, _st, n, Mc, L.inv.get());
+	YZ_LAUNCH(KGjExtract, std::min(148 * 8, ((n + 31) / 32) * ((n + 31) / 32)), 256, 0, _st, n, Mc, _gjOrig.get(), L.inv.get());
 }
 
 //--------------------------------------------------------------------------

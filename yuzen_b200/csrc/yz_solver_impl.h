@@ -10,6 +10,7 @@
 namespace yz {
 
 class Learned;
+struct GjPanel;
 template<class T> struct ClPlan;
 
 //  Scalars of one BiCGStab run, in device memory (written by the block that
@@ -186,9 +187,9 @@ private:
 	DBuf<double> _gtVal;
 	DBuf<int> _apPtr, _apCol;
 	DBuf<double> _apVal;
-	DBuf<double> _gj[2];          // [A | I] column-major, the panel multipliers
-	DBuf<double> _gjPiv;
-	DBuf<int> _gjRow;
+	DBuf<double> _gj[2];          // the direct level's slots column-major, the multipliers of two panels
+	DBuf<GjPanel> _gjPan;
+	DBuf<int> _gjOrig;
 	TryBackoff _offSpai;
 	//  hierarchy reuse (0: a new set-up every solve, the reference's way)
 	int _amgReuse = 0, _sinceBuild = 0, _freshIters = 0, _rebuilds = 0;
