@@ -329,7 +329,8 @@ int yz_step_set_graph_loop(yz_step* st, int on);
  * each (-1: the library's default, level 2 or YZ_FUSE_FROM; 0: none),
  * coarse_lanes the lanes a row of the coarse levels' kernels (0: by the
  * level's mean row length; 1, 2, 4 or 8), fine_sweeps the post-smoothing
- * sweeps at the finest level (0: the default, 5 or YZ_FINE_SWEEPS; 1 to 8).
+ * sweeps at the finest level, a Chebyshev iteration (0: the default, 8 or
+ * YZ_FINE_SWEEPS; 1 to 8).
  * The launch shapes change the preconditioner by float rounding only, the
  * sweeps change it (a better one); the FP64 cycle, the reference's, is not
  * affected.  yuzen_b200.autotune picks them per instance size. */

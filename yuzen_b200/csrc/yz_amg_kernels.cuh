@@ -286,20 +286,55 @@ __global__ void KAssignSecond(int n, const int *__restrict__ ptr, const int *__r
 	}
 }
 
+//  M32: the float copy for the FP32 cycle (null: none).  lam (null: not
+//  wanted): by their bits, lam[0] the largest |m_i| sum_j |a_ij|, a bound of
+//  the spectral radius of M A, and lam[1] the least m_i sum_j a_ij (0 if
+//  negative) of the rows that are not a ghost's two entries -- the value
+//  of M A on the constant, the bottom of its spectrum where A is the identity
+//  plus a difference operator; lam[0] zero, lam[1] all ones before
 __global__ void KSpai0(int n, const int *__restrict__ ptr, const int *__restrict__ col,
-                       const double *__restrict__ val, double *__restrict__ M)
+                       const double *__restrict__ val, double *__restrict__ M, float *__restrict__ M32,
+                       unsigned long long *lam)
 {
+	unsigned long long most = 0, least = ~0ull;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
-		double num = 0.0, den = 0.0;
-		for(int k = ptr[i]; k < ptr[i + 1]; ++k)
+		const int st = ptr[i], ed = ptr[i + 1];
+		double num = 0.0, den = 0.0, sum = 0.0, all = 0.0;
+		for(int k = st; k < ed; ++k)
 		{
 			const double v = val[k];
 			den = den + v * v;
 			if(col[k] == i) num = num + v;
+			sum = sum + fabs(v);
+			all = all + v;
 		}
-		M[i] = (1.0 / den) * num;
+		const double m = (1.0 / den) * num;
+		M[i] = m;
+		if(M32) M32[i] = (float)m;
+		const unsigned long long b = (unsigned long long)__double_as_longlong(fabs(m * sum));
+		most = b > most ? b : most;
+		const unsigned long long a = (unsigned long long)__double_as_longlong(m * all > 0.0 ? m * all : 0.0);
+		if(ed - st > 2) least = a < least ? a : least;
 	}
+	if(!lam) return;
+	for(int off = 16; off >= 1; off >>= 1)
+	{
+		const unsigned long long u = __shfl_down_sync(0xffffffffu, most, off), d = __shfl_down_sync(0xffffffffu, least, off);
+		most = u > most ? u : most;
+		least = d < least ? d : least;
+	}
+	if((threadIdx.x & 31) == 0) { atomicMax(lam, most); atomicMin(lam + 1, least); }
+}
+
+//  The weight of a Chebyshev step on [max(lo, hi / r), hi]: ck the cosine of
+//  the step's root, ir = 1 / r
+__host__ __device__ __forceinline__ double ChebWeight(const double *lam, double ck, double ir)
+{
+	const double hi = lam[0], lo0 = lam[1];
+	double lo = hi * ir;
+	if(lo0 > lo && lo0 < hi) lo = lo0;
+	return 1.0 / (0.5 * ((hi + lo) - (hi - lo) * ck));
 }
 
 //  damped Jacobi as a preconditioner: m_i = 0.72 * (1 / a_ii)
@@ -718,22 +753,24 @@ __global__ void KProlong(const int *__restrict__ halt, int n, const int *__restr
 	}
 }
 
-//  xout = x + m .* (f - A x)
-template<class T, class TF, class TX>
+//  xout = x + w m .* (f - A x); w 1, or (W) a step of the Chebyshev
+//  iteration on the bounds KSpai0 left
+template<class T, class TF, class TX, bool W = false>
 __global__ void KPostSmooth(const int *__restrict__ halt, int n, const int *__restrict__ ptr,
                             const int *__restrict__ sellOff, Sten sn, const int *__restrict__ col,
                             const T *__restrict__ val, const T *__restrict__ M, const TF *__restrict__ f,
-                            const T *__restrict__ x, TX *__restrict__ xout)
+                            const T *__restrict__ x, TX *__restrict__ xout, const double *__restrict__ lam, double ck, double ir)
 {
 	PdlEntry();
 	if(halt && *halt) return;
+	const T w = W ? (T)ChebWeight(lam, ck, ir) : T(1);
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		int st, len, sd;
 		RowRange(ptr, sellOff, i, st, len, sd);
 		const T s = RowSumSten(sn, i, st, len, sd, col, val, [&](int c) { return x[c]; });
 		const T t = (T)f[i] - s;
-		xout[i] = (TX)(x[i] + M[i] * t);
+		xout[i] = (TX)(x[i] + (W ? w * M[i] : M[i]) * t);
 	}
 }
 

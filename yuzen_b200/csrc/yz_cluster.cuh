@@ -52,6 +52,8 @@ template<class T>
 struct ClPlan
 {
 	int count, sweeps;                       // levels; the finest level's post-smoothing sweeps
+	double root[8], ratio;                   // and, for more than one, their Chebyshev roots (ChebWeight)
+	const double *lam;
 	const int *so;                           // the finest level's SELL-32 slices
 	Sten sn;
 	ClLevel<T> lv[kClMaxLevels];             // lv[0].val, .col: SELL-32
@@ -262,7 +264,7 @@ __device__ __forceinline__ void ClDense(const ClWho &who, int n, const T *inv, c
 	{
 		const T *row = inv + (size_t)i * n;
 		T s = T(0);
-		#pragma unroll 1
+#pragma unroll 1
 		for(int j0 = lane; j0 < n; j0 += 256)
 		{
 			T a[8], b[8];
@@ -366,18 +368,21 @@ __device__ __forceinline__ void ClCycle(const ClWho &who, const ClPlan<T> &P, co
 	T *xin = L.xt, *xo = L.x;
 	for(int k = 1; k < P.sweeps; ++k)
 	{
+		const T wk = (T)ChebWeight(P.lam, P.root[k - 1], P.ratio);
 		YZ_CL_FINE(i, n)
 		{
 			const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return xin[c]; });
-			xo[i] = xin[i] + __ldg(L.M + i) * ((T)r[i] - s);
+			xo[i] = xin[i] + wk * __ldg(L.M + i) * ((T)r[i] - s);
 		}
 		ClBarrier();
 		T *u = xin; xin = xo; xo = u;
 	}
+	const T w = P.sweeps > 1 ? (T)ChebWeight(P.lam, P.root[P.sweeps - 1], P.ratio) : T(1);
 	YZ_CL_FINE(i, n)
 	{
 		const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return xin[c]; });
-		z[i] = (double)(xin[i] + __ldg(L.M + i) * ((T)r[i] - s));
+		const T m = __ldg(L.M + i);
+		z[i] = (double)(xin[i] + (P.sweeps > 1 ? w * m : m) * ((T)r[i] - s));
 	}
 	ClBarrier();
 }

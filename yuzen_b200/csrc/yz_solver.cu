@@ -331,6 +331,7 @@ Solver::Solver(int device, cudaStream_t stream) : _device(device)
 	YZ_CUDA(cudaEventCreateWithFlags(&_evRing[0], cudaEventDisableTiming));
 	YZ_CUDA(cudaEventCreateWithFlags(&_evRing[1], cudaEventDisableTiming));
 	_sc.reserve(1);
+	_lam.reserve(2);
 	_counters.reserve(16);
 	YZ_CUDA(cudaMemsetAsync(_counters.get(), 0, 16 * sizeof(unsigned), _st));
 	_flags.reserve(8);
@@ -609,7 +610,9 @@ void Solver::BuildHierarchy(int coarseEnough)
 		          _state.get(), _iso.get(), _rootId.get(), _first.get());
 		YZ_LAUNCH(KAssignSecond, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _iptr.get(), _icol.get(),
 		          _iso.get(), _first.get(), L.agg.get());
-		YZ_LAUNCH(KSpai0, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), L.M.get());
+		unsigned long long *lam = l == 0 && _precision != YZ_PREC_FP64 ? reinterpret_cast<unsigned long long *>(_lam.get()) : nullptr;
+		if(lam) ClearBounds();
+		YZ_LAUNCH(KSpai0, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), L.M.get(), nullptr, lam);
 		L.nc = nc;
 		if(nc == 0) break;		// nothing to coarsen: this level is smoothed only
 		//  P
@@ -681,7 +684,7 @@ void Solver::Cycle(size_t l, const double *f, double *x)
 		Level &C = *_levels[l + 1];
 		YZ_LAUNCH(KPreSmoothResidual, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
 		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, x, L.t.get());
-		if(l > 0 || !LaunchCoarse<double>())
+		if(!LaunchCoarse<double>(l))
 		{
 			YZ_LAUNCH(KRestrict, GridFor((long long)C.n * 4, kB), kB, 0, _st, Halt(), C.n, L.rptr.get(), L.rcol.get(),
 			          L.rval.get(), L.t.get(), C.f.get());
@@ -689,13 +692,13 @@ void Solver::Cycle(size_t l, const double *f, double *x)
 		}
 		YZ_LAUNCH(KProlong, g, kB, 0, _st, Halt(), n, L.pptr.get(), L.pcol.get(), L.pval.get(), C.x.get(), x, L.xt.get());
 		YZ_LAUNCH(KPostSmooth, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
-		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x);
+		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x, nullptr, 0.0, 0.0);
 	}
 	else
 	{
 		YZ_LAUNCH(KPreSmooth, g, kB, 0, _st, Halt(), n, L.M.get(), f, L.xt.get());
 		YZ_LAUNCH(KPostSmooth, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
-		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x);
+		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x, nullptr, 0.0, 0.0);
 	}
 }
 
@@ -724,7 +727,7 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 		          val, L.M32.get(), f, L.x32.get(), L.t32.get());
 		LaunchCoarseCycle();
 		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
-		          L.M32.get(), f, L.xt32.get(), x);
+		          L.M32.get(), f, L.xt32.get(), x, nullptr, 0.0, 0.0);
 		return;
 	}
 	if(l + 1 < _nlev)
@@ -750,7 +753,7 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 		if(la == 1)
 			YZ_LAUNCH_PDL((KPreSmoothResidual<float, TF, float>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
 			          val, L.M32.get(), f, L.x32.get(), L.t32.get());
-		if(l > 0 || !LaunchCoarse<float>())
+		if(!LaunchCoarse<float>(l))
 		{
 			YZ_LAUNCH_PDL(KRestrict<float>, GridFor((long long)C.n * 4, kB), kB, 0, _st, Halt(), C.n, L.rptr.get(), L.rcol.get(),
 			              L.rval32.get(), L.t32.get(), C.f32.get());
@@ -767,26 +770,30 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 		}
 		if(la == 1)
 		{
-			//  FineSweeps() - 1 more SPAI0 sweeps at the finest level before
-			//  the last, float to float (x32 and xt32 in turn)
+			//  the finest level's sweeps: the Chebyshev iteration, float to
+			//  float (x32 and xt32 in turn) but for the last
 			const float *xin = L.xt32.get();
-			if(l == 0)
-				for(int k = 1; k < FineSweeps(); ++k)
-				{
-					float *xo = (xin == L.xt32.get()) ? L.x32.get() : L.xt32.get();
-					YZ_LAUNCH_PDL((KPostSmooth<float, TF, float>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
-					          val, L.M32.get(), f, xin, xo);
-					xin = xo;
-				}
-			YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
-			          L.M32.get(), f, xin, x);
+			const int K = l == 0 ? FineSweeps() : 1;
+			for(int k = 0; k + 1 < K; ++k)
+			{
+				float *xo = (xin == L.xt32.get()) ? L.x32.get() : L.xt32.get();
+				YZ_LAUNCH_PDL((KPostSmooth<float, TF, float, true>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
+				              val, L.M32.get(), f, xin, xo, _lam.get(), SweepRoot(k, K), kSweepRatio);
+				xin = xo;
+			}
+			if(K > 1)
+				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX, true>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
+				              L.M32.get(), f, xin, x, _lam.get(), SweepRoot(K - 1, K), kSweepRatio);
+			else
+				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
+				              L.M32.get(), f, xin, x, nullptr, 0.0, 0.0);
 		}
 	}
 	else
 	{
 		YZ_LAUNCH_PDL((KPreSmooth<float, TF, float>), g, kB, 0, _st, Halt(), n, L.M32.get(), f, L.xt32.get());
 		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val, L.M32.get(), f,
-		          L.xt32.get(), x);
+		          L.xt32.get(), x, nullptr, 0.0, 0.0);
 	}
 }
 
@@ -873,16 +880,30 @@ int Solver::FusedFrom() const
 	return _fuseFrom > 0 ? _fuseFrom : k;
 }
 
-//  The FP32 cycle's post-smoothing sweeps at the finest level (the FP64
-//  cycle keeps the reference's one).  SPAI0 smooths the film's fourth-order
-//  rows weakly: on the 512^2 film 5 sweeps cut the BiCGStab iterations from
-//  760 to 408 over 12 steps and the step from 11.7 to 9.7 ms (1: 85, 3: 99,
-//  4: 101, 5: 102-103, 6-8: 101-102 steps/s).  YZ_FINE_SWEEPS or SetTuning
-//  override the default, 5.
+//  The FP32 cycle's post-smoothing at the finest level (the FP64 cycle keeps
+//  the reference's one sweep): FineSweeps() sweeps x + w_k m (f - A x), the
+//  weights those of the Chebyshev iteration for the part of the spectrum of
+//  M A above a ratio of its bound.  Sweeps of weight 1 damp both ends of it
+//  weakly (at the bound, about 1.9, by 0.9 a sweep).  The lower end is the
+//  bound over 20, or the operator's own bottom where that is higher (KSpai0:
+//  a film with a short step is well conditioned, and reaching below its
+//  spectrum wastes sweeps: 9 iterations became 13).  Solves of one step,
+//  iterations and ms, 5 sweeps of weight 1 against 8 Chebyshev sweeps: 512^2
+//  all-physics 25, 5.0 -> 10, 2.7; 301^2 38, 7.1 -> 17, 4.5; 1024^2 162, 86 ->
+//  124, 80; 224^2 levelling 13, 2.1 -> 9, 1.5.  Five Chebyshev sweeps: 15, 3.3;
+//  24, 5.0; 145, 76; 13, 2.0.  YZ_FINE_SWEEPS or SetTuning override the 8.
+double Solver::SweepRoot(int k, int K) { return std::cos(3.14159265358979323846 * (2 * k + 1) / (2.0 * K)); }
+
+void Solver::ClearBounds()
+{
+	YZ_CUDA(cudaMemsetAsync(_lam.get(), 0, sizeof(double), _st));
+	YZ_CUDA(cudaMemsetAsync(_lam.get() + 1, 0xff, sizeof(double), _st));
+}
+
 int Solver::FineSweeps() const
 {
 	static const char *env = std::getenv("YZ_FINE_SWEEPS");
-	static const int k = env ? std::max(1, std::min(8, std::atoi(env))) : 5;
+	static const int k = env ? std::max(1, std::min(8, std::atoi(env))) : 8;
 	return _fineSweeps > 0 ? _fineSweeps : k;
 }
 
@@ -1103,14 +1124,19 @@ template<auto kernel> int ClusterBlocks(int device)
 }
 } // namespace
 
-template<class T> bool Solver::FillPlan(ClPlan<T> &P) const
+//  the hierarchy from level l0 on
+template<class T> bool Solver::FillPlan(ClPlan<T> &P, size_t l0) const
 {
-	if(_nlev > (size_t)kClMaxLevels) return false;
-	P.count = (int)_nlev;
+	if(_nlev - l0 > (size_t)kClMaxLevels) return false;
+	P.count = (int)(_nlev - l0);
 	P.sweeps = std::is_same<T, float>::value ? FineSweeps() : 1;
+	P.lam = _lam.get();
+	P.ratio = kSweepRatio;
+	for(int k = 0; k < P.sweeps; ++k) P.root[k] = SweepRoot(k, P.sweeps);
 	P.so = _sellOff.get();
 	P.sn = _sten;
-	for(size_t l = 0; l < _nlev; ++l) FillLevel(P.lv[l], *_levels[l], l + 1 == _nlev);
+	for(size_t l = l0; l < _nlev; ++l) FillLevel(P.lv[l - l0], *_levels[l], l + 1 == _nlev);
+	if(l0 > 0) return true;
 	P.lv[0].col = _sellCol.get();
 	if constexpr(std::is_same<T, double>::value) P.lv[0].val = _sellVal.get();
 	else P.lv[0].val = _sellVal32.get();
@@ -1124,7 +1150,7 @@ template<class V, class T> bool Solver::LaunchLoop(int kind, const V *val)
 	const int size = ClusterBlocks<KLoopCluster<V, T>>(_device);
 	if(!size) return false;
 	ClPlan<T> P = {};
-	if(kind == kPrecAmg && !FillPlan(P)) return false;
+	if(kind == kPrecAmg && !FillPlan(P, 0)) return false;
 	ClSystem<V> S;
 	S.n = _n;
 	S.ptr = _levels[0]->ptr.get(); S.so = _sellOff.get(); S.col = _sellCol.get();
@@ -1140,7 +1166,7 @@ template<class V, class T> bool Solver::LaunchLoop(int kind, const V *val)
 
 bool Solver::ClusterRun(int kind)
 {
-	if(kind == kPrecLearned || _n > ClusterRows()) return false;
+	if(kind == kPrecLearned || _n > ClusterRows() || ShapesSet()) return false;
 	if(_precision == YZ_PREC_FP32_MATRIX) return LaunchLoop<float, float>(kind, _sellVal32.get());
 	if(_precision == YZ_PREC_FP32_CYCLE) return LaunchLoop<double, float>(kind, _sellVal.get());
 	return LaunchLoop<double, double>(kind, _sellVal.get());
@@ -1157,18 +1183,23 @@ int Solver::ClusterRows() const
 	static const char *env = std::getenv("YZ_CLUSTER_ROWS");
 	static const int set = env ? std::min(std::atoi(env), kClMaxChunks * kRChunk) : -1;
 	if(set >= 0) return set;
-	return _precision == YZ_PREC_FP64 ? 20000 : 14000;
+	return _precision == YZ_PREC_FP64 ? 20000 : 11000;
 }
 
-//  the levels below the finest in one launch of a cluster
-template<class T> bool Solver::LaunchCoarse()
+//  The levels below level l -- its restriction, the V-cycle from l + 1 down
+//  -- in one launch of a cluster, where l + 1 is the first level of at most
+//  YZ_CLUSTER_COARSE rows (8,000: the 6,052 rows and 67,600 above them of a ConcZ film take
+//  106 ms a step so and 114 with the line at 3,000; the 55,000 of a 1024^2
+//  film's first coarse level took twice the separate launches' time).
+template<class T> bool Solver::LaunchCoarse(size_t l)
 {
 	static const char *env = std::getenv("YZ_CLUSTER_COARSE");
-	if(env && env[0] == '0') return false;
-	ClPlan<T> P = {};
-	if(_nlev < 2 || !FillPlan(P)) return false;
+	static const int most = env ? std::atoi(env) : 8000;
+	if(l + 1 >= _nlev || _levels[l + 1]->n > most || ShapesSet()) return false;
 	const int size = ClusterBlocks<KCoarseCluster<T>>(_device);
 	if(!size) return false;
+	ClPlan<T> P = {};
+	if(!FillPlan(P, l)) return false;
 	LaunchCluster(KCoarseCluster<T>, size, _st, "KCoarseCluster", Halt(), P);
 	return true;
 }
@@ -1242,7 +1273,7 @@ void Solver::RunIterations(int kind)
 		++hooks;
 	};
 	if(collect) _zs.reserve((size_t)_n);
-	if(graphOff || TimingActive() || collect || (!_graphLoop && (kind == kPrecLearned || _n > ClusterRows())))
+	if(graphOff || TimingActive() || collect || (!_graphLoop && (kind == kPrecLearned || _n > ClusterRows() || ShapesSet())))
 	{
 		//  one iteration kept in flight: the state after iteration k is
 		//  copied to pinned memory and read while iteration k+1 runs; the
@@ -1453,7 +1484,7 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 	if(set.conc && set.precondition == 2 && _offSpai.Try())
 	{
 		YZ_PROF("lin.fallback.conc", _st);
-		YZ_LAUNCH(KSpai0, g, kB, 0, _st, n, L0.ptr.get(), L0.col.get(), L0.val.get(), _m.get());
+		YZ_LAUNCH(KSpai0, g, kB, 0, _st, n, L0.ptr.get(), L0.col.get(), L0.val.get(), _m.get(), nullptr, nullptr);
 		if(!BiCGStab(kPrecDiag, tryIter, set.epsilon, it, err)) err = 1e300;
 		if(err <= set.epsilon) { done = true; _offSpai.Converged(); }
 		else
@@ -1535,13 +1566,10 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 						Level &F = *_levels[0];
 						if(!F.direct)
 						{
-							YZ_LAUNCH(KSpai0, g, kB, 0, _st, n, F.ptr.get(), F.col.get(), F.val.get(), F.M.get());
-							if(fp32)
-							{
-								RoundList one;
-								one.count = 1; one.src[0] = F.M.get(); one.dst[0] = F.M32.get(); one.n[0] = n;
-								YZ_LAUNCH(KRoundToFloat, GridFor(n, kB), kB, 0, _st, one);
-							}
+							unsigned long long *lam = fp32 ? reinterpret_cast<unsigned long long *>(_lam.get()) : nullptr;
+							if(lam) ClearBounds();
+							YZ_LAUNCH(KSpai0, g, kB, 0, _st, n, F.ptr.get(), F.col.get(), F.val.get(), F.M.get(),
+							          fp32 ? F.M32.get() : nullptr, lam);
 						}
 						++_sinceBuild;
 					}

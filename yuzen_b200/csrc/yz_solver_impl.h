@@ -105,9 +105,9 @@ private:
 	template<class TF, class TX> void Cycle32(size_t l, const TF *f, TX *x);
 	int LanesFor(long long nnz, int n) const;
 	//  the runs and coarse levels that one cluster takes (yz_cluster.cuh)
-	template<class T> bool FillPlan(ClPlan<T> &P) const;
+	template<class T> bool FillPlan(ClPlan<T> &P, size_t l0) const;
 	template<class V, class T> bool LaunchLoop(int kind, const V *val);
-	template<class T> bool LaunchCoarse();
+	template<class T> bool LaunchCoarse(size_t l);
 	bool ClusterRun(int kind);
 	int ClusterRows() const;
 	bool CoarseCycleOn() const;
@@ -123,6 +123,14 @@ private:
 	//  KUpFused); past the deepest level: none
 	int FusedFrom() const;
 	int FineSweeps() const;
+	//  the Chebyshev sweeps: the cosine of root k of K, the assumed ratio of
+	//  the least to the largest eigenvalue
+	static double SweepRoot(int k, int K);
+	static constexpr double kSweepRatio = 1.0 / 20.0;
+	void ClearBounds();
+	//  launch shapes asked for (SetTuning) on the FP32 cycle's separate
+	//  launches: the one-cluster forms stand back
+	bool ShapesSet() const { return _precision != YZ_PREC_FP64 && (_fuseFrom >= 0 || _coarseLanes > 0); }
 	void CoarseDown(int lanes, int nc, const Level &L, const float *f, float *fc);
 	void CoarseUp(int lanes, const Level &L, const float *f, const float *xc, float *x);
 	const int *Halt() const { return &_sc.get()->state; }
@@ -173,6 +181,7 @@ private:
 	int _partBlocks = 1;
 	DBuf<unsigned> _counters;
 	DBuf<Scal> _sc;
+	DBuf<double> _lam;          // bounds of the spectrum of M A at the finest level (the FP32 cycle's; KSpai0)
 	Scal *_hsc = nullptr;
 	int *_hint = nullptr;      // pinned: totals and flags read back together
 	Scal *_hring = nullptr;    // pinned: the state after the last two iterations
