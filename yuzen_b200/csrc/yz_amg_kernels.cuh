@@ -150,82 +150,97 @@ __global__ void KDiag(int n, const int *__restrict__ ptr, const int *__restrict_
 	}
 }
 
+//  strong[k]: entry k of A is a strong connection; cnt: of every row, its
+//  strong connections either way (a row that both holds and is held counts
+//  twice: every use of the lists is a max or a min over them)
 __global__ void KStrength(int n, const int *__restrict__ ptr, const int *__restrict__ col,
                           const double *__restrict__ val, const double *__restrict__ dia, double eps2,
-                          unsigned char *__restrict__ strong, int *__restrict__ icnt)
+                          unsigned char *__restrict__ strong, int *__restrict__ cnt)
 {
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		const double e = eps2 * dia[i];
+		int out = 0;
 		for(int k = ptr[i]; k < ptr[i + 1]; ++k)
 		{
 			const int c = col[k];
 			const double v = val[k];
 			const bool s = (c != i) && (e * dia[c] < v * v);
 			strong[k] = s ? 1 : 0;
-			if(s) atomicAdd(&icnt[c], 1);
+			if(s) { ++out; atomicAdd(&cnt[c], 1); }
 		}
+		if(out) atomicAdd(&cnt[i], out);
 	}
 }
 
-//  in-neighbours (rows that hold this one strongly); the order inside a list
-//  is free, every later use is a max or a min over it
+//  the strong neighbours of every row, held and holding, in one list (in any
+//  order): the rounds and the aggregation then read one list instead of
+//  scanning a row's flags beside a second one
 __global__ void KFillIn(int n, const int *__restrict__ ptr, const int *__restrict__ col,
-                        const unsigned char *__restrict__ strong, int *__restrict__ ifill, int *__restrict__ icol)
-{
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-		for(int k = ptr[i]; k < ptr[i + 1]; ++k)
-			if(strong[k]) icol[atomicAdd(&ifill[col[k]], 1)] = i;
-}
-
-__global__ void KMisInit(int n, const int *__restrict__ ptr, const unsigned char *__restrict__ strong,
-                         const int *__restrict__ iptr, int *__restrict__ state, unsigned char *__restrict__ iso)
+                        const unsigned char *__restrict__ strong, int *__restrict__ fill, int *__restrict__ nbr)
 {
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
-		bool any = iptr[i + 1] > iptr[i];
-		for(int k = ptr[i]; k < ptr[i + 1] && !any; ++k) any = strong[k] != 0;
-		iso[i] = any ? 0 : 1;
-		state[i] = any ? kUndecided : kOut;
+		int out = 0;
+		for(int k = ptr[i]; k < ptr[i + 1]; ++k)
+			if(strong[k]) { ++out; nbr[atomicAdd(&fill[col[k]], 1)] = i; }
+		if(!out) continue;
+		int at = atomicAdd(&fill[i], out);
+		for(int k = ptr[i]; k < ptr[i + 1]; ++k)
+			if(strong[k]) nbr[at++] = col[k];
 	}
 }
 
 //  The rounds of the distance-2 independent set.  Round r reads the count of
-//  undecided rows u[r & 1] (0: the set is complete, the round does nothing),
-//  takes the largest key within distance 2 (KMisMax twice), and KMisUpdate
-//  decides the rows, writes the keys of the next round over the maxima it
-//  has read and counts the rows still undecided into u[(r + 1) & 1], which
-//  the round's first KMisMax has zeroed.
-__global__ void KMisPack(int n, const int *__restrict__ state, unsigned long long *__restrict__ T0, int *__restrict__ undecided)
+//  undecided rows u[r & 1] (0: the set is complete, the round does nothing):
+//  KMisMax takes the largest key next to each row and zeroes u[(r + 1) & 1],
+//  KMisUpdate the largest within distance 2, decides the row, writes its key of
+//  the next round and counts the rows still undecided into u[(r + 1) & 1].
+__global__ void KMisInit(int n, const int *__restrict__ nptr, int *__restrict__ state, unsigned char *__restrict__ iso,
+                         unsigned long long *__restrict__ T0, int *__restrict__ undecided)
 {
 	int cnt = 0;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
-		T0[i] = PackKey(state[i], i);
-		cnt += (state[i] == kUndecided);
+		const bool any = nptr[i + 1] > nptr[i];
+		iso[i] = any ? 0 : 1;
+		state[i] = any ? kUndecided : kOut;
+		T0[i] = PackKey(any ? kUndecided : kOut, i);
+		cnt += any;
 	}
 	for(int off = 16; off >= 1; off >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, off);
 	if((threadIdx.x & 31) == 0 && cnt) atomicAdd(undecided, cnt);
 }
 
-__global__ void KMisMax(int n, const int *__restrict__ ptr, const int *__restrict__ col,
-                        const unsigned char *__restrict__ strong, const int *__restrict__ iptr,
-                        const int *__restrict__ icol, const unsigned long long *__restrict__ Tin,
-                        unsigned long long *__restrict__ Tout, const int *__restrict__ undecided, int *zero)
+__device__ __forceinline__ unsigned long long MisMaxRow(int i, const int *__restrict__ nptr, const int *__restrict__ nbr,
+                                                        const unsigned long long *__restrict__ T)
 {
-	if(zero && blockIdx.x == 0 && threadIdx.x == 0) *zero = 0;
-	if(*undecided == 0) return;
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+	unsigned long long m = T[i];
+	const int ed = nptr[i + 1];
+	for(int k = nptr[i]; k < ed; k += 4)
 	{
-		unsigned long long m = Tin[i];
-		for(int k = ptr[i]; k < ptr[i + 1]; ++k) if(strong[k]) { const unsigned long long u = Tin[col[k]]; m = u > m ? u : m; }
-		for(int k = iptr[i]; k < iptr[i + 1]; ++k) { const unsigned long long u = Tin[icol[k]]; m = u > m ? u : m; }
-		Tout[i] = m;
+		unsigned long long u[4];
+#pragma unroll
+		for(int j = 0; j < 4; ++j) u[j] = k + j < ed ? T[nbr[k + j]] : 0ull;
+#pragma unroll
+		for(int j = 0; j < 4; ++j) m = u[j] > m ? u[j] : m;
 	}
+	return m;
 }
 
-__global__ void KMisUpdate(int n, int *__restrict__ state, unsigned long long *__restrict__ T2, const int *__restrict__ undecided,
-                           int *__restrict__ nextUndecided)
+__global__ void KMisMax(int n, const int *__restrict__ nptr, const int *__restrict__ nbr,
+                        const unsigned long long *__restrict__ Tin, unsigned long long *__restrict__ Tout,
+                        const int *__restrict__ undecided, int *zero)
+{
+	if(blockIdx.x == 0 && threadIdx.x == 0) *zero = 0;
+	if(*undecided == 0) return;
+	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+		Tout[i] = MisMaxRow(i, nptr, nbr, Tin);
+}
+
+__global__ void KMisUpdate(int n, const int *__restrict__ nptr, const int *__restrict__ nbr,
+                           const unsigned long long *__restrict__ T1, int *__restrict__ state,
+                           unsigned long long *__restrict__ T0, const int *__restrict__ undecided, int *__restrict__ next)
 {
 	if(*undecided == 0) return;
 	int cnt = 0;
@@ -234,16 +249,15 @@ __global__ void KMisUpdate(int n, int *__restrict__ state, unsigned long long *_
 		int st = state[i];
 		if(st == kUndecided)
 		{
-			const unsigned long long t = T2[i];
+			const unsigned long long t = MisMaxRow(i, nptr, nbr, T1);
 			if((int)(uint32_t)(t & 0xffffffffull) == i) st = kIn;
 			else if((int)(t >> 62) == kIn) st = kOut;
-			state[i] = st;
+			if(st != kUndecided) { state[i] = st; T0[i] = PackKey(st, i); }
 		}
-		T2[i] = PackKey(st, i);
 		cnt += (st == kUndecided);
 	}
 	for(int off = 16; off >= 1; off >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, off);
-	if((threadIdx.x & 31) == 0 && cnt) atomicAdd(nextUndecided, cnt);
+	if((threadIdx.x & 31) == 0 && cnt) atomicAdd(next, cnt);
 }
 
 __global__ void KRootFlags(int n, const int *__restrict__ state, int *__restrict__ flag)
@@ -251,37 +265,30 @@ __global__ void KRootFlags(int n, const int *__restrict__ state, int *__restrict
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) flag[i] = state[i] == kIn ? 1 : 0;
 }
 
-__global__ void KAssignFirst(int n, const int *__restrict__ ptr, const int *__restrict__ col,
-                             const unsigned char *__restrict__ strong, const int *__restrict__ iptr,
-                             const int *__restrict__ icol, const int *__restrict__ state,
-                             const unsigned char *__restrict__ iso, const int *__restrict__ rootId, int *__restrict__ first)
+__global__ void KAssignFirst(int n, const int *__restrict__ nptr, const int *__restrict__ nbr,
+                             const int *__restrict__ state, const unsigned char *__restrict__ iso,
+                             const int *__restrict__ rootId, int *__restrict__ first)
 {
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		if(state[i] == kIn) { first[i] = rootId[i]; continue; }
 		if(iso[i]) { first[i] = -1; continue; }
 		int best = -1;
-		for(int k = ptr[i]; k < ptr[i + 1]; ++k)
-			if(strong[k]) { const int j = col[k]; if(state[j] == kIn && (best < 0 || rootId[j] < best)) best = rootId[j]; }
-		for(int k = iptr[i]; k < iptr[i + 1]; ++k)
-		{ const int j = icol[k]; if(state[j] == kIn && (best < 0 || rootId[j] < best)) best = rootId[j]; }
+		for(int k = nptr[i]; k < nptr[i + 1]; ++k)
+		{ const int j = nbr[k]; if(state[j] == kIn && (best < 0 || rootId[j] < best)) best = rootId[j]; }
 		first[i] = best;
 	}
 }
 
-__global__ void KAssignSecond(int n, const int *__restrict__ ptr, const int *__restrict__ col,
-                              const unsigned char *__restrict__ strong, const int *__restrict__ iptr,
-                              const int *__restrict__ icol, const unsigned char *__restrict__ iso,
-                              const int *__restrict__ first, int *__restrict__ agg)
+__global__ void KAssignSecond(int n, const int *__restrict__ nptr, const int *__restrict__ nbr,
+                              const unsigned char *__restrict__ iso, const int *__restrict__ first, int *__restrict__ agg)
 {
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		if(first[i] >= 0 || iso[i]) { agg[i] = first[i]; continue; }
 		int best = -1;
-		for(int k = ptr[i]; k < ptr[i + 1]; ++k)
-			if(strong[k]) { const int f = first[col[k]]; if(f >= 0 && (best < 0 || f < best)) best = f; }
-		for(int k = iptr[i]; k < iptr[i + 1]; ++k)
-		{ const int f = first[icol[k]]; if(f >= 0 && (best < 0 || f < best)) best = f; }
+		for(int k = nptr[i]; k < nptr[i + 1]; ++k)
+		{ const int f = first[nbr[k]]; if(f >= 0 && (best < 0 || f < best)) best = f; }
 		agg[i] = best;
 	}
 }
@@ -416,8 +423,9 @@ __global__ void KPFill(int n, const int *__restrict__ ptr, const int *__restrict
 }
 
 //  R = P^T: counts per column, atomic fill, then each row sorted by fine row
-__global__ void KColCount(int nnz, const int *__restrict__ pcol, int *__restrict__ cnt)
+__global__ void KColCount(const int *__restrict__ total, const int *__restrict__ pcol, int *__restrict__ cnt)
 {
+	const int nnz = *total;
 	for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += gridDim.x * blockDim.x) atomicAdd(&cnt[pcol[k]], 1);
 }
 
@@ -559,7 +567,7 @@ __global__ void __launch_bounds__(256) KGemmWarp(int nx, const int *__restrict__
                                                  const int *__restrict__ ycol, const double *__restrict__ yval,
                                                  int *__restrict__ cnt, const int *__restrict__ cptr,
                                                  int *__restrict__ ccol, double *__restrict__ cval,
-                                                 int *__restrict__ overflow)
+                                                 int *__restrict__ overflow, bool ystage = false)
 {
 	constexpr int W = 8;
 	__shared__ int scol[W][CAP];
@@ -581,7 +589,8 @@ __global__ void __launch_bounds__(256) KGemmWarp(int nx, const int *__restrict__
 			const bool av = xk < xe;
 			const int kk = av ? xcol[xk] : 0;
 			const double xvv = (FILL && av) ? xval[xk] : 0.0;
-			const int ys = av ? yptr[kk] : 0, ye = av ? yptr[kk + 1] : 0;
+			//  (ystage: Y's rows staged, row k at k CAP with yptr[k] entries)
+			const int ys = !av ? 0 : ystage ? kk * CAP : yptr[kk], ye = !av ? 0 : ystage ? ys + yptr[kk] : yptr[kk + 1];
 			const int cntx = (xe - xb < 32) ? xe - xb : 32;
 		for(int jx = 0; jx < cntx && !over; ++jx)
 		{

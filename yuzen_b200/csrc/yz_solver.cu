@@ -442,6 +442,8 @@ void Solver::SetPattern(int n, int nnz, const int *rowptr, const int *scol, cons
 	_nlev = 1;
 	Level &L0 = *_levels[0];
 	L0.n = n; L0.nnz = nnz;
+	L0.most = 0;
+	for(int i = 0; i < n; ++i) L0.most = std::max(L0.most, _hptr[(size_t)i + 1] - _hptr[(size_t)i]);
 	L0.ptr.upload(rowptr, (size_t)n + 1, _st);
 	L0.col.upload(scol, (size_t)nnz, _st);
 	L0.val.reserve((size_t)nnz);
@@ -454,7 +456,7 @@ void Solver::SetPattern(int n, int nnz, const int *rowptr, const int *scol, cons
 	_part.reserve((size_t)2 * _partBlocks);
 	//  set-up scratch, sized by the finest level
 	_dia.reserve((size_t)n); _strong.reserve((size_t)nnz); _icnt.reserve((size_t)n + 1);
-	_iptr.reserve((size_t)n + 1); _icol.reserve((size_t)nnz); _ifill.reserve((size_t)n + 1);
+	_iptr.reserve((size_t)n + 1); _icol.reserve(2 * (size_t)nnz); _ifill.reserve((size_t)n + 1);
 	_state.reserve((size_t)n); _iso.reserve((size_t)n);
 	_T0.reserve((size_t)n); _T1.reserve((size_t)n);
 	_flag.reserve((size_t)n + 1); _rootId.reserve((size_t)n + 1); _first.reserve((size_t)n);
@@ -491,37 +493,34 @@ int Solver::ScanCounts(const int *cnt, int *out, int n, const int *flag, int *fl
 	return _hint[0];
 }
 
-//  C = X Y: one warp per row with room for 64 distinct columns (KGemmWarp),
-//  each row computed once into a staging slot and moved to its place after
-//  the counts are scanned; the thread-per-row kernels with kRowCap where a
-//  row needs more; returns nnz(C)
-int Solver::Gemm(int nx, const int *xptr, const int *xcol, const double *xval, const int *yptr, const int *ycol,
-                 const double *yval, DBuf<int> &cptr, DBuf<int> &ccol, DBuf<double> &cval)
+//  C = X Y with up to kRowCap distinct columns a row, a thread a row; returns
+//  nnz(C)
+int Solver::WideGemm(int nx, const int *xptr, const int *xcol, const double *xval, const int *yptr, const int *ycol,
+                     const double *yval, DBuf<int> &cptr, DBuf<int> &ccol, DBuf<double> &cval)
 {
 	int *overflow = _flags.get() + 1;
 	const int g = GridFor(nx, 128);
-	const int gw = GridFor((long long)nx * 32, 256, 148 * 64);
 	YZ_CUDA(cudaMemsetAsync(overflow, 0, sizeof(int), _st));
-	//  one pass: every row into a staging slot of 64, with its count
-	_gtCol.reserve((size_t)nx * 64); _gtVal.reserve((size_t)nx * 64);
-	YZ_LAUNCH((KGemmWarp<64, true>), gw, 256, 0, _st, nx, xptr, xcol, xval, yptr, ycol, yval, _cnt.get(), nullptr,
-	          _gtCol.get(), _gtVal.get(), overflow);
+	YZ_LAUNCH(KGemmCount<kRowCap>, g, 128, 0, _st, nx, xptr, xcol, yptr, ycol, _cnt.get(), overflow);
 	cptr.reserve((size_t)nx + 1);
 	int ovf = 0;
-	int nnz = ScanCounts(_cnt.get(), cptr.get(), nx, overflow, &ovf);
-	const bool wide = ovf != 0;
-	if(wide)
-	{
-		YZ_CUDA(cudaMemsetAsync(overflow, 0, sizeof(int), _st));
-		YZ_LAUNCH(KGemmCount<kRowCap>, g, 128, 0, _st, nx, xptr, xcol, yptr, ycol, _cnt.get(), overflow);
-		nnz = ScanCounts(_cnt.get(), cptr.get(), nx);
-		if(ReadInt(overflow)) throw CudaError("AMG set-up: a row of a product gathered more than 256 distinct columns");
-	}
+	const int nnz = ScanCounts(_cnt.get(), cptr.get(), nx, overflow, &ovf);
+	if(ovf) throw CudaError("AMG set-up: a row of a product gathered more than 256 distinct columns");
 	ccol.reserve((size_t)nnz); cval.reserve((size_t)nnz);
-	if(wide) YZ_LAUNCH(KGemmFill<kRowCap>, g, 128, 0, _st, nx, xptr, xcol, xval, yptr, ycol, yval, cptr.get(), ccol.get(), cval.get());
-	else YZ_LAUNCH(KGemmCompact<64>, GridFor((long long)nx * 64, 256, 148 * 64), 256, 0, _st, nx, cptr.get(),
-	               _gtCol.get(), _gtVal.get(), ccol.get(), cval.get());
+	YZ_LAUNCH(KGemmFill<kRowCap>, g, 128, 0, _st, nx, xptr, xcol, xval, yptr, ycol, yval, cptr.get(), ccol.get(), cval.get());
 	return nnz;
+}
+
+template<int CAP> void Solver::CountP(Level &L, int *overflow)
+{
+	YZ_LAUNCH(KPCount<CAP>, GridFor(L.n, kB), kB, 0, _st, L.n, L.ptr.get(), L.col.get(), _strong.get(), L.agg.get(), _cnt.get(),
+	          overflow);
+}
+
+template<int CAP> void Solver::FillP(Level &L)
+{
+	YZ_LAUNCH(KPFill<CAP>, GridFor(L.n, kB), kB, 0, _st, L.n, L.ptr.get(), L.col.get(), L.val.get(), _strong.get(), L.agg.get(),
+	          L.pptr.get(), L.pcol.get(), L.pval.get());
 }
 
 //  The dense inverse of the direct level (yz_gj.cuh): a launch a panel of
@@ -579,7 +578,8 @@ void Solver::BuildHierarchy(int coarseEnough)
 			DirectInverse(L);
 			break;
 		}
-		//  strength
+		//  strength, and the list of every row's strong neighbours
+		_strong.reserve((size_t)nnz); _icol.reserve(2 * (size_t)nnz);
 		YZ_LAUNCH(KDiag, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _dia.get());
 		YZ_CUDA(cudaMemsetAsync(_icnt.get(), 0, ((size_t)n + 1) * sizeof(int), _st));
 		YZ_LAUNCH(KStrength, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _dia.get(), eps * eps,
@@ -588,76 +588,96 @@ void Solver::BuildHierarchy(int coarseEnough)
 		ScanExclusive(_icnt.get(), _iptr.get(), n, _scan.get(), _st);
 		YZ_CUDA(cudaMemcpyAsync(_ifill.get(), _iptr.get(), (size_t)n * sizeof(int), cudaMemcpyDeviceToDevice, _st));
 		YZ_LAUNCH(KFillIn, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _ifill.get(), _icol.get());
-		//  MIS-2 (at most 64 rounds, as the oracle)
-		YZ_LAUNCH(KMisInit, g, kB, 0, _st, n, L.ptr.get(), _strong.get(), _iptr.get(), _state.get(), _iso.get());
+		//  MIS-2 (at most 64 rounds, as the oracle): eight rounds, nearly always
+		//  enough, are queued before the host reads how many rows are left
 		int *undec = _flags.get() + 4;		// two counters, by round parity
 		YZ_CUDA(cudaMemsetAsync(undec, 0, 2 * sizeof(int), _st));
-		YZ_LAUNCH(KMisPack, g, kB, 0, _st, n, _state.get(), _T0.get(), undec);
-		for(int round = 0; round < 64; ++round)
+		YZ_LAUNCH(KMisInit, g, kB, 0, _st, n, _iptr.get(), _state.get(), _iso.get(), _T0.get(), undec);
+		int nc = 0;
+		for(int round = 0; round < 64;)
 		{
-			int *u = undec + (round & 1), *un = undec + ((round + 1) & 1);
-			YZ_LAUNCH(KMisMax, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _iptr.get(), _icol.get(),
-			          _T0.get(), _T1.get(), u, un);
-			YZ_LAUNCH(KMisMax, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _iptr.get(), _icol.get(),
-			          _T1.get(), _T0.get(), u, nullptr);
-			YZ_LAUNCH(KMisUpdate, g, kB, 0, _st, n, _state.get(), _T0.get(), u, un);
-			if((round & 3) == 3 && ReadInt(un) == 0) break;
+			for(int end = round + (round ? 4 : 8); round < end; ++round)
+			{
+				int *u = undec + (round & 1), *un = undec + ((round + 1) & 1);
+				YZ_LAUNCH(KMisMax, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _T0.get(), _T1.get(), u, un);
+				YZ_LAUNCH(KMisUpdate, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _T1.get(), _state.get(), _T0.get(), u, un);
+			}
+			//  the aggregates' roots, with the count of rows left
+			YZ_LAUNCH(KRootFlags, g, kB, 0, _st, n, _state.get(), _flag.get());
+			int left = 0;
+			nc = ScanCounts(_flag.get(), _rootId.get(), n, undec + (round & 1), &left);
+			if(left == 0) break;
 		}
-		//  aggregates
-		YZ_LAUNCH(KRootFlags, g, kB, 0, _st, n, _state.get(), _flag.get());
-		const int nc = ScanCounts(_flag.get(), _rootId.get(), n);
-		YZ_LAUNCH(KAssignFirst, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _iptr.get(), _icol.get(),
-		          _state.get(), _iso.get(), _rootId.get(), _first.get());
-		YZ_LAUNCH(KAssignSecond, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _iptr.get(), _icol.get(),
-		          _iso.get(), _first.get(), L.agg.get());
+		YZ_LAUNCH(KAssignFirst, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _state.get(), _iso.get(), _rootId.get(),
+		          _first.get());
+		YZ_LAUNCH(KAssignSecond, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _iso.get(), _first.get(), L.agg.get());
 		unsigned long long *lam = l == 0 && _precision != YZ_PREC_FP64 ? reinterpret_cast<unsigned long long *>(_lam.get()) : nullptr;
 		if(lam) ClearBounds();
 		YZ_LAUNCH(KSpai0, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), L.M.get(), nullptr, lam);
 		L.nc = nc;
 		if(nc == 0) break;		// nothing to coarsen: this level is smoothed only
-		//  P
-		int *overflow = _flags.get() + 1;
-		YZ_CUDA(cudaMemsetAsync(overflow, 0, sizeof(int), _st));
-		YZ_LAUNCH(KPCount<32>, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), L.agg.get(), _cnt.get(),
-		          overflow);
-		L.pptr.reserve((size_t)n + 1);
-		int ovfP = 0;
-		L.pnnz = ScanCounts(_cnt.get(), L.pptr.get(), n, overflow, &ovfP);
-		const bool wideP = ovfP != 0;
-		if(wideP)
-		{
-			YZ_CUDA(cudaMemsetAsync(overflow, 0, sizeof(int), _st));
-			YZ_LAUNCH(KPCount<kRowCap>, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), L.agg.get(),
-			          _cnt.get(), overflow);
-			L.pnnz = ScanCounts(_cnt.get(), L.pptr.get(), n);
-			if(ReadInt(overflow)) throw CudaError("AMG set-up: a row of P gathered more than 256 distinct aggregates");
-		}
-		L.pcol.reserve((size_t)L.pnnz); L.pval.reserve((size_t)L.pnnz);
-		if(wideP)
-			YZ_LAUNCH(KPFill<kRowCap>, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _strong.get(), L.agg.get(),
-			          L.pptr.get(), L.pcol.get(), L.pval.get());
-		else
-			YZ_LAUNCH(KPFill<32>, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _strong.get(), L.agg.get(),
-			          L.pptr.get(), L.pcol.get(), L.pval.get());
+		if(_levels.size() <= l + 1) _levels.emplace_back(new Level());
+		_nlev = l + 2;
+		Level &C = *_levels[l + 1];
+		C.n = nc;
+		//  P, whose row holds at most a row of A's entries: room for that many
+		//  columns a row and nnz(A) in all, so that the sizes need not be read
+		//  before the products (a read empties the queue: 20 us of it idle)
+		const bool cap32 = L.most <= 32, cap64 = L.most <= 64;
+		int *overflow = _flags.get() + 1;		// [1] the products', [2] P's
+		YZ_CUDA(cudaMemsetAsync(overflow, 0, 2 * sizeof(int), _st));
+		L.pptr.reserve((size_t)n + 1); L.pcol.reserve((size_t)nnz); L.pval.reserve((size_t)nnz);
+		if(cap32) CountP<32>(L, overflow + 1);
+		else if(cap64) CountP<64>(L, overflow + 1);
+		else CountP<kRowCap>(L, overflow + 1);
+		ScanExclusive(_cnt.get(), L.pptr.get(), n, _scan.get(), _st);
+		if(cap32) FillP<32>(L);
+		else if(cap64) FillP<64>(L);
+		else FillP<kRowCap>(L);
 		//  R = P^T
-		L.rptr.reserve((size_t)nc + 1); L.rcol.reserve((size_t)L.pnnz); L.rval.reserve((size_t)L.pnnz);
+		L.rptr.reserve((size_t)nc + 1); L.rcol.reserve((size_t)nnz); L.rval.reserve((size_t)nnz);
 		YZ_CUDA(cudaMemsetAsync(_cnt.get(), 0, ((size_t)nc + 1) * sizeof(int), _st));
-		YZ_LAUNCH(KColCount, GridFor(L.pnnz, kB), kB, 0, _st, L.pnnz, L.pcol.get(), _cnt.get());
+		YZ_LAUNCH(KColCount, gz, kB, 0, _st, L.pptr.get() + n, L.pcol.get(), _cnt.get());
 		ScanExclusive(_cnt.get(), L.rptr.get(), nc, _scan.get(), _st);
 		YZ_CUDA(cudaMemcpyAsync(_ifill.get(), L.rptr.get(), (size_t)nc * sizeof(int), cudaMemcpyDeviceToDevice, _st));
 		YZ_LAUNCH(KTransposeFill, g, kB, 0, _st, n, L.pptr.get(), L.pcol.get(), L.pval.get(), _ifill.get(),
 		          L.rcol.get(), L.rval.get());
 		YZ_LAUNCH(KRowSort, GridFor((long long)nc * 32, 256, 148 * 64), 256, 0, _st, nc, L.rptr.get(), L.rcol.get(),
 		          L.rval.get());
-		//  AP, then A_c = R (AP)
-		Gemm(n, L.ptr.get(), L.col.get(), L.val.get(), L.pptr.get(), L.pcol.get(), L.pval.get(), _apPtr, _apCol, _apVal);
-		if(_levels.size() <= l + 1) _levels.emplace_back(new Level());
-		_nlev = l + 2;
-		Level &C = *_levels[l + 1];
-		Level &F = *_levels[l];
-		C.n = nc;
-		C.nnz = Gemm(nc, F.rptr.get(), F.rcol.get(), F.rval.get(), _apPtr.get(), _apCol.get(), _apVal.get(), C.ptr, C.col,
-		             C.val);
+		//  AP staged, 64 places a row, then A_c = R (AP) from the staged rows
+		_apCnt.reserve((size_t)n); _apCol.reserve((size_t)n * 64); _apVal.reserve((size_t)n * 64);
+		_gtCol.reserve((size_t)nc * 64); _gtVal.reserve((size_t)nc * 64);
+		YZ_LAUNCH((KGemmWarp<64, true>), GridFor((long long)n * 32, 256, 148 * 64), 256, 0, _st, n, L.ptr.get(), L.col.get(),
+		          L.val.get(), L.pptr.get(), L.pcol.get(), L.pval.get(), _apCnt.get(), nullptr, _apCol.get(), _apVal.get(),
+		          overflow, false);
+		YZ_LAUNCH((KGemmWarp<64, true>), GridFor((long long)nc * 32, 256, 148 * 64), 256, 0, _st, nc, L.rptr.get(),
+		          L.rcol.get(), L.rval.get(), _apCnt.get(), _apCol.get(), _apVal.get(), _cnt.get(), nullptr, _gtCol.get(),
+		          _gtVal.get(), overflow, true);
+		C.ptr.reserve((size_t)nc + 1);
+		ScanExclusive(_cnt.get(), C.ptr.get(), nc, _scan.get(), _st);
+		//  the level's sizes in one round trip
+		YZ_CUDA(cudaMemcpyAsync(_hint, C.ptr.get() + nc, sizeof(int), cudaMemcpyDeviceToHost, _st));
+		YZ_CUDA(cudaMemcpyAsync(_hint + 1, L.pptr.get() + n, sizeof(int), cudaMemcpyDeviceToHost, _st));
+		YZ_CUDA(cudaMemcpyAsync(_hint + 2, overflow, 2 * sizeof(int), cudaMemcpyDeviceToHost, _st));
+		YZ_CUDA(cudaStreamSynchronize(_st));
+		C.nnz = _hint[0]; L.pnnz = _hint[1];
+		if(_hint[3]) throw CudaError("AMG set-up: a row of P gathered more than 256 distinct aggregates");
+		if(!_hint[2])
+		{
+			C.most = 64;
+			C.col.reserve((size_t)C.nnz); C.val.reserve((size_t)C.nnz);
+			YZ_LAUNCH(KGemmCompact<64>, GridFor((long long)nc * 64, 256, 148 * 64), 256, 0, _st, nc, C.ptr.get(),
+			          _gtCol.get(), _gtVal.get(), C.col.get(), C.val.get());
+		}
+		else
+		{
+			//  a row of a product has more than 64 columns: the thread-per-row
+			//  kernels
+			C.most = kRowCap;
+			WideGemm(n, L.ptr.get(), L.col.get(), L.val.get(), L.pptr.get(), L.pcol.get(), L.pval.get(), _apPtr, _apCol, _apVal);
+			C.nnz = WideGemm(nc, L.rptr.get(), L.rcol.get(), L.rval.get(), _apPtr.get(), _apCol.get(), _apVal.get(), C.ptr, C.col,
+			                 C.val);
+		}
 	}
 	_haveH = true;
 }

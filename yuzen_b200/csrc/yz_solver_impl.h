@@ -41,6 +41,7 @@ struct TryBackoff
 struct Level
 {
 	int n = 0, nnz = 0;
+	int most = 0;           // entries a row of A has at most
 	DBuf<int> ptr, col;
 	DBuf<double> val;
 	DBuf<double> M, f, x, t, xt;
@@ -153,8 +154,10 @@ private:
 	int ReadInt(const int *d);
 	void ReadScal();
 	int ScanCounts(const int *cnt, int *out, int n, const int *flag = nullptr, int *flagOut = nullptr);
-	int Gemm(int nx, const int *xptr, const int *xcol, const double *xval, const int *yptr, const int *ycol,
-	         const double *yval, DBuf<int> &cptr, DBuf<int> &ccol, DBuf<double> &cval);
+	int WideGemm(int nx, const int *xptr, const int *xcol, const double *xval, const int *yptr, const int *ycol,
+	             const double *yval, DBuf<int> &cptr, DBuf<int> &ccol, DBuf<double> &cval);
+	template<int CAP> void CountP(Level &L, int *overflow);
+	template<int CAP> void FillP(Level &L);
 	RedScratch Red(int site);
 
 	int _device;
@@ -194,7 +197,7 @@ private:
 	DBuf<unsigned long long> _T0, _T1;
 	DBuf<int> _gtCol;             // staged rows of a product (64 a row)
 	DBuf<double> _gtVal;
-	DBuf<int> _apPtr, _apCol;
+	DBuf<int> _apPtr, _apCnt, _apCol;
 	DBuf<double> _apVal;
 	DBuf<double> _gj[2];          // the direct level's slots column-major, the multipliers of two panels
 	DBuf<GjPanel> _gjPan;
