@@ -483,3 +483,41 @@ def test_chebyshev_sweeps_meet_the_tolerance(N, stiff, sweeps):
         return
     assert g[0] == 0, g[:3]
     assert _true_residual(d, g[3]) <= 2e-10
+
+
+def _hub_system(n: int, width: int, seed: int) -> dict:
+    """A diagonally dominant band of n rows with hub rows of `width` entries
+    tied to rows all over the system, so that rows of A, P and the coarse
+    product run past the short forms' slots (32 and 64 a row)."""
+    rng = np.random.default_rng(seed)
+    cols = [{i} | {j for j in (i - 40, i - 1, i + 1, i + 40) if 0 <= j < n} for i in range(n)]
+    for h in rng.choice(n, 8, replace=False).tolist():
+        for j in rng.choice(n, width, replace=False).tolist():
+            cols[h].add(j)
+            cols[j].add(h)
+    rows = [[i] + sorted(c - {i}) for i, c in enumerate(cols)]
+    rowptr = np.zeros(n + 1, np.int32)
+    rowptr[1:] = np.cumsum([len(r) for r in rows])
+    col = np.array([c for r in rows for c in r], np.int32)
+    own = np.repeat(np.arange(n), np.diff(rowptr))
+    val = -rng.uniform(0.5, 1.0, col.size)
+    val[rowptr[:-1]] = 0.0
+    val[rowptr[:-1]] = 0.01 - np.bincount(own, weights=val, minlength=n)
+    scol, ssrc = _systems.sorted_mirror(rowptr, col)
+    return {"n": n, "nnz": col.size, "rowptr": rowptr, "col": col, "sorted_col": scol, "sorted_src": ssrc,
+            "values": val, "rhs": rng.standard_normal(n), "x0": np.zeros(n), "precondition": 2, "scaling": 0,
+            "max_iteration": 200, "epsilon": 1e-10, "conc": 0}
+
+
+@pytest.mark.parametrize("width", [20, 26, 40, 59, 60, 120])
+def test_wide_rows_bitwise(width):
+    d = _hub_system(6400, width, width)
+    if width == 120:        # a row of A P gathers 256 columns and more: refused, as the interface states
+        with pytest.raises(yz.YzError, match="more than 256 distinct columns"):
+            gpu_solve(d)
+        return
+    g = gpu_solve(d)
+    o = _oracle.OracleSolver()
+    assert_same(g[:4], o.solve(d))
+    assert g[0] == 0
+    _levels_equal(g[4].levels(), o.levels())

@@ -42,9 +42,12 @@ __device__ __forceinline__ void RowRange(const int *__restrict__ ptr, const int 
 }
 
 //  sum_k val[e_k] * X(col[e_k]) over a row (e_k = st + k stride), from 0 in
-//  the row's order: the loads of four entries are issued together and the
-//  products then added one after the other, so the sum is the sequential
-//  one with four loads in flight instead of one.  T is the arithmetic (the
+//  the row's order: the loads of R entries are issued together, the last
+//  ones of a row under a predicate, and the products then added one after the
+//  other, so the sum is the sequential one and a row waits for two loads in
+//  turn per R entries.  (With the last len mod 4 entries one by one, the
+//  13-entry rows of a film's edges waited 9 times and held up their blocks:
+//  the smoother of 262,144 rows 7.8 us, now 6.8.)  T is the arithmetic (the
 //  type of the values): double everywhere but in the FP32 V-cycle.
 //  The values may be stored narrower than the arithmetic (float values in a
 //  double sum: the FP32-matrix SpMV); the arithmetic is that of X.
@@ -53,47 +56,65 @@ __device__ __forceinline__ auto RowSum(int st, int len, int sd, const int *__res
                                        XF xf) -> decltype(xf(0))
 {
 	using T = decltype(xf(0));
+	constexpr int R = 4;
 	T s = T(0);
-	int k = 0, e = st;
-	for(; k + 4 <= len; k += 4, e += 4 * sd)
+	for(int k = 0, e = st; k < len; k += R, e += R * sd)
 	{
-		const int c0 = col[e], c1 = col[e + sd], c2 = col[e + 2 * sd], c3 = col[e + 3 * sd];
-		const T v0 = (T)val[e], v1 = (T)val[e + sd], v2 = (T)val[e + 2 * sd], v3 = (T)val[e + 3 * sd];
-		const T x0 = xf(c0), x1 = xf(c1), x2 = xf(c2), x3 = xf(c3);
-		s = s + v0 * x0;
-		s = s + v1 * x1;
-		s = s + v2 * x2;
-		s = s + v3 * x3;
+		int c[R];
+		V v[R];
+		T x[R];
+#pragma unroll
+		for(int j = 0; j < R; ++j)
+		{
+			const bool on = k + j < len;
+			c[j] = on ? col[e + j * sd] : 0;
+			v[j] = on ? val[e + j * sd] : V(0);
+		}
+#pragma unroll
+		for(int j = 0; j < R; ++j) x[j] = k + j < len ? xf(c[j]) : T(0);
+#pragma unroll
+		for(int j = 0; j < R; ++j)
+			if(k + j < len) s = s + (T)v[j] * x[j];
 	}
-	for(; k < len; ++k, e += sd) s = s + (T)val[e] * xf(col[e]);
 	return s;
 }
 
-//  RowSum of row i of the finest level (SELL-32, entry k at st + 32 k).  A
-//  stencil row's loop is unrolled to the 16 entries a stencil may have, so
-//  that every offset is read from the kernel's parameters by a constant
-//  index; the sum is the same sequential one.
+//  RowSum of row i of a level; a stencil row's length and offsets come from
+//  the kernel's parameters (the loop is unrolled to the 16 entries a stencil
+//  may have, so every offset is read by a constant index), so that its values
+//  and x hang on no other read than the slice's flag and place.  The sum is
+//  the same sequential one.  Four entries at a time: eight take 40 to 64
+//  registers for 32 and a third of the warps, which is slower from 262,144
+//  rows (the smoother at 1,048,576 rows in float 18.2 for 17.1 us).
 template<class V, class XF>
-__device__ __forceinline__ auto RowSumSten(const Sten &sn, int i, int st, int len, int sd, const int *__restrict__ col,
+__device__ __forceinline__ auto RowSumSten(const Sten &sn, int i, const int *__restrict__ ptr,
+                                           const int *__restrict__ sellOff, const int *__restrict__ col,
                                            const V *__restrict__ val, XF xf) -> decltype(xf(0))
 {
 	using T = decltype(xf(0));
-	if(sn.slice && sn.slice[i >> 5])
+	int st, len, sd;
+	RowRange(ptr, sellOff, i, st, len, sd);
+	if(sn.slice)
 	{
-		T s = T(0);
-#pragma unroll
-		for(int k0 = 0; k0 < 16; k0 += 4)
+		if(sn.slice[i >> 5])
 		{
-			if(k0 >= len) break;
-			T v[4], xv[4];
+			const V *__restrict__ row = val + st;
+			T s = T(0);
 #pragma unroll
-			for(int j = 0; j < 4; ++j)
-				if(k0 + j < len) { v[j] = (T)val[st + (k0 + j) * sd]; xv[j] = xf(i + sn.off[k0 + j]); }
+			for(int k0 = 0; k0 < 16; k0 += 4)
+			{
+				if(k0 >= sn.len) break;
+				V v[4];
+				T xv[4];
 #pragma unroll
-			for(int j = 0; j < 4; ++j)
-				if(k0 + j < len) s = s + v[j] * xv[j];
+				for(int j = 0; j < 4; ++j)
+					if(k0 + j < sn.len) { v[j] = row[32 * (k0 + j)]; xv[j] = xf(i + sn.off[k0 + j]); }
+#pragma unroll
+				for(int j = 0; j < 4; ++j)
+					if(k0 + j < sn.len) s = s + (T)v[j] * xv[j];
+			}
+			return s;
 		}
-		return s;
 	}
 	return RowSum(st, len, sd, col, val, xf);
 }
@@ -590,18 +611,19 @@ __global__ void __launch_bounds__(256) KGemmWarp(int nx, const int *__restrict__
 			const int kk = av ? xcol[xk] : 0;
 			const double xvv = (FILL && av) ? xval[xk] : 0.0;
 			//  (ystage: Y's rows staged, row k at k CAP with yptr[k] entries)
-			const int ys = !av ? 0 : ystage ? kk * CAP : yptr[kk], ye = !av ? 0 : ystage ? ys + yptr[kk] : yptr[kk + 1];
+			const int ys = !av ? 0 : ystage ? kk : yptr[kk], yl = !av ? 0 : ystage ? yptr[kk] : yptr[kk + 1] - ys;
 			const int cntx = (xe - xb < 32) ? xe - xb : 32;
 		for(int jx = 0; jx < cntx && !over; ++jx)
 		{
-			const int y0 = __shfl_sync(0xffffffffu, ys, jx);
-			const int y1 = __shfl_sync(0xffffffffu, ye, jx);
+			const int yr = __shfl_sync(0xffffffffu, ys, jx);
+			const int y1 = __shfl_sync(0xffffffffu, yl, jx);
+			const long long y0 = ystage ? (long long)yr * CAP : (long long)yr;
 			const double xv = __shfl_sync(0xffffffffu, xvv, jx);
-			for(int base = y0; base < y1 && !over; base += 32)
+			for(int base = 0; base < y1 && !over; base += 32)
 			{
 				const int ky = base + lane;
 				const bool active = ky < y1;
-				const int j = active ? ycol[ky] : -1;
+				const int j = active ? ycol[y0 + ky] : -1;
 				int slot = -1;
 				if(active)
 					for(int q = 0; q < m; ++q) if(scol[w][q] == j) { slot = q; break; }
@@ -617,7 +639,7 @@ __global__ void __launch_bounds__(256) KGemmWarp(int nx, const int *__restrict__
 				}
 				m += add;
 				__syncwarp();
-				if(FILL && active) sval[w][slot] = sval[w][slot] + xv * yval[ky];
+				if(FILL && active) sval[w][slot] = sval[w][slot] + xv * yval[y0 + ky];
 				__syncwarp();
 			}
 		}
@@ -683,17 +705,16 @@ __global__ void KGemmCompact(int nx, const int *__restrict__ cptr, const int *__
 //  x = m .* f, t = f - A x (x of the neighbours recomputed as m_j * f_j)
 template<class T, class TF, class TX>
 __global__ void KPreSmoothResidual(const int *__restrict__ halt, int n, const int *__restrict__ ptr,
-                                   const int *__restrict__ sellOff, Sten sn, const int *__restrict__ col,
+                                   const int *__restrict__ sellOff, const __grid_constant__ Sten sn, const int *__restrict__ col,
                                    const T *__restrict__ val, const T *__restrict__ M, const TF *__restrict__ f,
                                    TX *__restrict__ x, T *__restrict__ t)
 {
 	PdlEntry();
 	if(halt && *halt) return;
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i < n)
 	{
-		int st, len, sd;
-		RowRange(ptr, sellOff, i, st, len, sd);
-		const T s = RowSumSten(sn, i, st, len, sd, col, val, [&](int c) { return M[c] * (T)f[c]; });
+		const T s = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return M[c] * (T)f[c]; });
 		const T fi = (T)f[i];
 		x[i] = (TX)(M[i] * fi);
 		t[i] = fi - s;
@@ -766,20 +787,19 @@ __global__ void KProlong(const int *__restrict__ halt, int n, const int *__restr
 //  iteration on the bounds KSpai0 left
 template<class T, class TF, class TX, bool W = false>
 __global__ void KPostSmooth(const int *__restrict__ halt, int n, const int *__restrict__ ptr,
-                            const int *__restrict__ sellOff, Sten sn, const int *__restrict__ col,
+                            const int *__restrict__ sellOff, const __grid_constant__ Sten sn, const int *__restrict__ col,
                             const T *__restrict__ val, const T *__restrict__ M, const TF *__restrict__ f,
                             const T *__restrict__ x, TX *__restrict__ xout, const double *__restrict__ lam, double ck, double ir)
 {
 	PdlEntry();
 	if(halt && *halt) return;
 	const T w = W ? (T)ChebWeight(lam, ck, ir) : T(1);
-	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i < n)
 	{
-		int st, len, sd;
-		RowRange(ptr, sellOff, i, st, len, sd);
-		const T s = RowSumSten(sn, i, st, len, sd, col, val, [&](int c) { return x[c]; });
-		const T t = (T)f[i] - s;
-		xout[i] = (TX)(x[i] + (W ? w * M[i] : M[i]) * t);
+		const T fi = (T)f[i], xi = x[i], mi = M[i];
+		const T s = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return x[c]; });
+		xout[i] = (TX)(xi + (W ? w * mi : mi) * (fi - s));
 	}
 }
 

@@ -175,9 +175,34 @@ struct DBuf
 //--------------------------------------------------------------------------
 constexpr int kRT = 256;
 constexpr int kRK = 1;
+constexpr int kRPer = 8;		// blocks an SM of the reducing kernels
 constexpr int kRChunk = kRT * kRK;
 
-inline int RedBlocks(int n) { const int nb = (n + kRChunk - 1) / kRChunk; return nb > 0 ? nb : 1; }
+__host__ __device__ inline int RedChunks(int n) { return n > 0 ? (n + kRChunk - 1) / kRChunk : 1; }
+inline int RedBlocks(int n) { return RedChunks(n); }
+
+//  The blocks that share the chunks (ChunkFold): at most the 8 of 256 threads that an SM holds, and
+//  of those as many as give each the same number of chunks.
+inline int RedGrid(int n)
+{
+	const int nb = RedBlocks(n), per = (nb + 148 * kRPer - 1) / (148 * kRPer);
+	return (nb + per - 1) / per;
+}
+
+//  The tree over 256 values v[0..255] in shared memory, by one warp: the folds
+//  at 128, 64 and 32 of lane t read v[t + 32 w] of the 8 warps, so one warp
+//  makes them without a barrier between (the same sums in the same order as
+//  the pairwise fold).  Result valid in lane 0.
+__device__ __forceinline__ double LaneTree(const double *v, int t)
+{
+	double u[8];
+#pragma unroll
+	for(int w = 0; w < 8; ++w) u[w] = v[t + 32 * w];
+	double s = ((u[0] + u[4]) + (u[2] + u[6])) + ((u[1] + u[5]) + (u[3] + u[7]));
+#pragma unroll
+	for(int off = 16; off >= 1; off >>= 1) s = s + __shfl_down_sync(0xffffffffu, s, off);
+	return s;
+}
 
 //  Fold Q values per thread over a block of 256 (same order as Tree256).
 //  sh: Q*256 doubles of shared memory.  Result valid in thread 0.
@@ -188,26 +213,10 @@ __device__ __forceinline__ void BlockTree(double (&a)[Q], double *sh)
 #pragma unroll
 	for(int q = 0; q < Q; ++q) sh[q * kRT + t] = a[q];
 	__syncthreads();
-#pragma unroll
-	for(int off = kRT / 2; off >= 32; off >>= 1)
-	{
-		if(t < off)
-		{
-#pragma unroll
-			for(int q = 0; q < Q; ++q) sh[q * kRT + t] = sh[q * kRT + t] + sh[q * kRT + t + off];
-		}
-		__syncthreads();
-	}
 	if(t < 32)
 	{
 #pragma unroll
-		for(int q = 0; q < Q; ++q)
-		{
-			double v = sh[q * kRT + t];
-#pragma unroll
-			for(int off = 16; off >= 1; off >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, off);
-			a[q] = v;
-		}
+		for(int q = 0; q < Q; ++q) a[q] = LaneTree(sh + q * kRT, t);
 	}
 }
 
@@ -219,19 +228,19 @@ struct RedScratch
 	int maxBlocks;
 };
 
-//  Called by every block after its threads hold their per-thread sums a[q]:
-//  writes the block's partials; the last block to arrive folds them all and
-//  returns true with the totals in tot[q] (valid in every thread of it).
+//  The end of a grid's reduction: every block calls it after its threads'
+//  partials are written; the last block to arrive folds the `chunks` partials
+//  of each q and returns true with the totals in tot[q] (valid in every
+//  thread of it).  sh: Q*256 doubles that no thread reads any more after a
+//  barrier.
 template<int Q>
-__device__ __forceinline__ bool GridFold(double (&a)[Q], double *sh, const RedScratch rs, double (&tot)[Q])
+__device__ __forceinline__ bool GridLast(int chunks, double *sh, const RedScratch rs, double (&tot)[Q])
 {
 	__shared__ bool amLast;
-	BlockTree<Q>(a, sh);
+	__shared__ double bc[Q];
 	const int t = threadIdx.x;
 	if(t == 0)
 	{
-#pragma unroll
-		for(int q = 0; q < Q; ++q) rs.part[q * rs.maxBlocks + blockIdx.x] = a[q];
 		__threadfence();
 		const unsigned prev = atomicAdd(rs.counter, 1u);
 		amLast = (prev == gridDim.x - 1);
@@ -243,13 +252,20 @@ __device__ __forceinline__ bool GridFold(double (&a)[Q], double *sh, const RedSc
 #pragma unroll
 	for(int q = 0; q < Q; ++q)
 	{
+		//  eight loads in flight: the block is alone, so their latency is the time
 		double s = 0.0;
-		for(int j = t; j < (int)gridDim.x; j += kRT) s = s + __ldcg(&rs.part[q * rs.maxBlocks + j]);
+		for(int j = t; j < chunks; j += 8 * kRT)
+		{
+			double p[8];
+#pragma unroll
+			for(int u = 0; u < 8; ++u) p[u] = j + u * kRT < chunks ? __ldcg(&rs.part[q * rs.maxBlocks + j + u * kRT]) : 0.0;
+#pragma unroll
+			for(int u = 0; u < 8; ++u)
+				if(j + u * kRT < chunks) s = s + p[u];
+		}
 		b[q] = s;
 	}
-	__syncthreads();
 	BlockTree<Q>(b, sh);
-	__shared__ double bc[Q];
 	if(t == 0)
 	{
 #pragma unroll
@@ -261,6 +277,55 @@ __device__ __forceinline__ bool GridFold(double (&a)[Q], double *sh, const RedSc
 	for(int q = 0; q < Q; ++q) tot[q] = bc[q];
 	return true;
 }
+
+//  Called by every block of a grid of one block a chunk after its threads
+//  hold their per-thread sums a[q]: writes the block's partials, then GridLast.
+template<int Q>
+__device__ __forceinline__ bool GridFold(double (&a)[Q], double *sh, const RedScratch rs, double (&tot)[Q])
+{
+	BlockTree<Q>(a, sh);
+	if(threadIdx.x == 0)
+	{
+#pragma unroll
+		for(int q = 0; q < Q; ++q) rs.part[q * rs.maxBlocks + blockIdx.x] = a[q];
+	}
+	return GridLast<Q>((int)gridDim.x, sh, rs, tot);
+}
+
+//  One chunk's sums in a kernel whose grid of RedGrid(n) blocks shares the
+//  chunks (block b takes b, b + G, ...; c is the block's k-th): the block's
+//  values a[q] into shared memory, in two halves by turns, and one warp, k mod
+//  8, writes the chunk's partials while the others go on to the next chunk.
+//  The sums are the same whatever G is.  One barrier a chunk, and one fence
+//  and one atomic a block in GridLast (after a barrier) rather than one a
+//  chunk: at 1,048,576 rows the update of x and r went from 16.7 to 12.5 us,
+//  that of s from 12.4 to 9.4.  sh: 2*Q*256 doubles.
+//  The products with the matrix keep a block a chunk (GridFold): in a loop
+//  over chunks the compiler holds the row's 13 addresses across the turns,
+//  which at 32 registers spills (262,144 rows: 12.2 against 8.4 us), and
+//  fewer blocks an SM with more registers are slower too (10.4 to 11.2).
+template<int Q>
+__device__ __forceinline__ void ChunkFold(const double (&a)[Q], double *sh, int k, int c, const RedScratch rs)
+{
+	const int t = threadIdx.x;
+	double *v = sh + (k & 1) * Q * kRT;
+#pragma unroll
+	for(int q = 0; q < Q; ++q) v[q * kRT + t] = a[q];
+	__syncthreads();
+	if((t >> 5) == (k & 7))
+	{
+#pragma unroll
+		for(int q = 0; q < Q; ++q)
+		{
+			const double s = LaneTree(v + q * kRT, t & 31);
+			if((t & 31) == 0) rs.part[q * rs.maxBlocks + c] = s;
+		}
+	}
+}
+
+//  the loop of such a kernel: row i of chunk c, the block's k-th
+#define YZ_CHUNKS(n) for(int c_ = blockIdx.x, k_ = 0; c_ < RedChunks(n); c_ += gridDim.x, ++k_)
+#define YZ_CHUNK_ROW (c_ * kRChunk + (int)threadIdx.x)
 
 //--------------------------------------------------------------------------
 //  exclusive scan of n ints into out[0..n] (out[n] = total); integer, so

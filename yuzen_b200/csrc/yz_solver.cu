@@ -28,33 +28,29 @@ namespace yz {
 
 //==========================================================================
 //  Krylov kernels: element-wise updates fused with the dot products they
-//  feed, all on the chunk mapping of the reduction tree (block b, thread t:
-//  elements b*4096 + k*256 + t).  Scalars live in device memory (Scal).
+//  feed, all on the chunk mapping of the reduction tree (ChunkFold).  Scalars live in device memory (Scal).
 //==========================================================================
-#define YZ_CHUNK_LOOP(i)                                                          \
-	for(int kk_ = 0, i = blockIdx.x * kRChunk + threadIdx.x; kk_ < kRK; ++kk_, i += kRT)
 
 //  r = b - A x;  bb = b.b, rr = r.r, rho0 = r.r (rh = r)
 template<class V>
-__global__ void __launch_bounds__(kRT, 8) KBInit(int n, const int *__restrict__ ptr, const int *__restrict__ sellOff, Sten sn, const int *__restrict__ col,
+__global__ void __launch_bounds__(kRT, kRPer) KBInit(int n, const int *__restrict__ ptr, const int *__restrict__ sellOff, const __grid_constant__ Sten sn, const int *__restrict__ col,
                        const V *__restrict__ val, const double *__restrict__ b,
                        const double *__restrict__ x, double *__restrict__ r, double *__restrict__ rh,
                        RedScratch rs, Scal *sc)
 {
 	__shared__ double sh[2 * kRT];
+	double tot[2];
 	double a[2] = {0.0, 0.0};
-	YZ_CHUNK_LOOP(i)
+	const int i = blockIdx.x * kRT + threadIdx.x;
+	if(i < n)
 	{
-		if(i >= n) break;
-		int st, len, sd;
-		RowRange(ptr, sellOff, i, st, len, sd);
-		const double s = RowSumSten(sn, i, st, len, sd, col, val, [&](int c) { return x[c]; });
-		const double ri = b[i] - s;
+		const double bi = b[i];
+		const double s = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return x[c]; });
+		const double ri = bi - s;
 		r[i] = ri; rh[i] = ri;
-		a[0] = a[0] + b[i] * b[i];
+		a[0] = a[0] + bi * bi;
 		a[1] = a[1] + ri * ri;
 	}
-	double tot[2];
 	if(GridFold<2>(a, sh, rs, tot) && threadIdx.x == 0)
 	{
 		sc->normb = sqrt(tot[0]);
@@ -87,45 +83,50 @@ __global__ void KPUpdate(int n, const double *__restrict__ r, const double *__re
 
 //  v = A ph; alpha = rho / (rh . v)
 template<class V>
-__global__ void __launch_bounds__(kRT, 8) KSpmvAlpha(int n, const int *__restrict__ ptr, const int *__restrict__ sellOff, Sten sn,
+__global__ void __launch_bounds__(kRT, kRPer) KSpmvAlpha(int n, const int *__restrict__ ptr, const int *__restrict__ sellOff, Sten sn,
                            const int *__restrict__ col, const V *__restrict__ val, const double *__restrict__ ph,
                            const double *__restrict__ rh, double *__restrict__ v, RedScratch rs, Scal *sc)
 {
 	PdlEntry();
 	if(sc->state != kRun) return;
 	__shared__ double sh[kRT];
-	double a[1] = {0.0};
-	YZ_CHUNK_LOOP(i)
-	{
-		if(i >= n) break;
-		int st, len, sd;
-		RowRange(ptr, sellOff, i, st, len, sd);
-		const double s = RowSumSten(sn, i, st, len, sd, col, val, [&](int c) { return ph[c]; });
-		v[i] = s;
-		a[0] = a[0] + rh[i] * s;
-	}
+	const double rho = sc->rho;
 	double tot[1];
-	if(GridFold<1>(a, sh, rs, tot) && threadIdx.x == 0) sc->alpha = sc->rho / tot[0];
+	double a[1] = {0.0};
+	const int i = blockIdx.x * kRT + threadIdx.x;
+	if(i < n)
+	{
+		const double ri = rh[i];
+		const double s = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return ph[c]; });
+		v[i] = s;
+		a[0] = a[0] + ri * s;
+	}
+	if(GridFold<1>(a, sh, rs, tot) && threadIdx.x == 0) sc->alpha = rho / tot[0];
 }
 
 //  s = r - alpha v; res = |s|
-__global__ void KSUpdate(int n, const double *__restrict__ r, const double *__restrict__ v,
+__global__ void __launch_bounds__(kRT, kRPer) KSUpdate(int n, const double *__restrict__ r, const double *__restrict__ v,
                          double *__restrict__ s, RedScratch rs, Scal *sc)
 {
 	PdlEntry();
 	if(sc->state != kRun) return;
-	__shared__ double sh[kRT];
+	__shared__ double sh[2 * kRT];
 	const double alpha = sc->alpha;
-	double a[1] = {0.0};
-	YZ_CHUNK_LOOP(i)
-	{
-		if(i >= n) break;
-		const double si = r[i] - alpha * v[i];
-		s[i] = si;
-		a[0] = a[0] + si * si;
-	}
 	double tot[1];
-	if(GridFold<1>(a, sh, rs, tot) && threadIdx.x == 0)
+	YZ_CHUNKS(n)
+	{
+		double a[1] = {0.0};
+		const int i = YZ_CHUNK_ROW;
+		if(i < n)
+		{
+			const double si = r[i] - alpha * v[i];
+			s[i] = si;
+			a[0] = a[0] + si * si;
+		}
+		ChunkFold<1>(a, sh, k_, c_, rs);
+	}
+	__syncthreads();
+	if(GridLast<1>(RedChunks(n), sh, rs, tot) && threadIdx.x == 0)
 	{
 		const double res = sqrt(tot[0]);
 		sc->res = res;
@@ -137,25 +138,24 @@ __global__ void KSUpdate(int n, const double *__restrict__ r, const double *__re
 
 //  t = A sh; omega = (t . s) / (t . t)
 template<class V>
-__global__ void __launch_bounds__(kRT, 8) KSpmvOmega(int n, const int *__restrict__ ptr, const int *__restrict__ sellOff, Sten sn,
+__global__ void __launch_bounds__(kRT, kRPer) KSpmvOmega(int n, const int *__restrict__ ptr, const int *__restrict__ sellOff, Sten sn,
                            const int *__restrict__ col, const V *__restrict__ val, const double *__restrict__ sh_,
                            const double *__restrict__ s, double *__restrict__ t, RedScratch rs, Scal *sc)
 {
 	PdlEntry();
 	if(sc->state != kRun) return;
 	__shared__ double sh[2 * kRT];
+	double tot[2];
 	double a[2] = {0.0, 0.0};
-	YZ_CHUNK_LOOP(i)
+	const int i = blockIdx.x * kRT + threadIdx.x;
+	if(i < n)
 	{
-		if(i >= n) break;
-		int st, len, sd;
-		RowRange(ptr, sellOff, i, st, len, sd);
-		const double u = RowSumSten(sn, i, st, len, sd, col, val, [&](int c) { return sh_[c]; });
+		const double si = s[i];
+		const double u = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return sh_[c]; });
 		t[i] = u;
 		a[0] = a[0] + u * u;
-		a[1] = a[1] + u * s[i];
+		a[1] = a[1] + u * si;
 	}
-	double tot[2];
 	if(GridFold<2>(a, sh, rs, tot) && threadIdx.x == 0) sc->omega = tot[1] / tot[0];
 }
 
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kRT, 8) KSpmvOmega(int n, const int *__restric
 //  After a half-step exit (KSUpdate set kConvHalf, the rest of the iteration
 //  did nothing): x = x + alpha ph instead; the iteration's end turns the
 //  state into kConv, so that no later kernel repeats it.
-__global__ void KXRUpdate(int n, const double *__restrict__ ph, const double *__restrict__ shat,
+__global__ void __launch_bounds__(kRT, kRPer) KXRUpdate(int n, const double *__restrict__ ph, const double *__restrict__ shat,
                           const double *__restrict__ s, const double *__restrict__ t,
                           const double *__restrict__ rh, double *__restrict__ x, double *__restrict__ r,
                           RedScratch rs, Scal *sc)
@@ -173,28 +173,29 @@ __global__ void KXRUpdate(int n, const double *__restrict__ ph, const double *__
 	if(state == kConvHalf)
 	{
 		const double alpha = sc->alpha;
-		YZ_CHUNK_LOOP(i)
-		{
-			if(i >= n) break;
-			x[i] = x[i] + alpha * ph[i];
-		}
+		for(int i = blockIdx.x * kRT + threadIdx.x; i < n; i += gridDim.x * kRT) x[i] = x[i] + alpha * ph[i];
 		return;
 	}
 	if(state != kRun) return;
-	__shared__ double sh[2 * kRT];
+	__shared__ double sh[4 * kRT];
 	const double alpha = sc->alpha, omega = sc->omega;
-	double a[2] = {0.0, 0.0};
-	YZ_CHUNK_LOOP(i)
-	{
-		if(i >= n) break;
-		x[i] = (x[i] + alpha * ph[i]) + omega * shat[i];
-		const double ri = s[i] - omega * t[i];
-		r[i] = ri;
-		a[0] = a[0] + ri * ri;
-		a[1] = a[1] + rh[i] * ri;
-	}
 	double tot[2];
-	if(GridFold<2>(a, sh, rs, tot) && threadIdx.x == 0)
+	YZ_CHUNKS(n)
+	{
+		double a[2] = {0.0, 0.0};
+		const int i = YZ_CHUNK_ROW;
+		if(i < n)
+		{
+			x[i] = (x[i] + alpha * ph[i]) + omega * shat[i];
+			const double ri = s[i] - omega * t[i];
+			r[i] = ri;
+			a[0] = a[0] + ri * ri;
+			a[1] = a[1] + rh[i] * ri;
+		}
+		ChunkFold<2>(a, sh, k_, c_, rs);
+	}
+	__syncthreads();
+	if(GridLast<2>(RedChunks(n), sh, rs, tot) && threadIdx.x == 0)
 	{
 		const double res = sqrt(tot[0]);
 		sc->res = res;
@@ -256,20 +257,23 @@ __global__ void KFill(int n, double v, double *__restrict__ x)
 }
 
 //  the deterministic dot product on its own (for the parity tests)
-__global__ void KDot(int n, const double *__restrict__ x, const double *__restrict__ y, RedScratch rs, double *out)
+__global__ void __launch_bounds__(kRT, kRPer) KDot(int n, const double *__restrict__ x, const double *__restrict__ y, RedScratch rs, double *out)
 {
-	__shared__ double sh[kRT];
-	double a[1] = {0.0};
-	YZ_CHUNK_LOOP(i)
-	{
-		if(i >= n) break;
-		a[0] = a[0] + x[i] * y[i];
-	}
+	__shared__ double sh[2 * kRT];
 	double tot[1];
-	if(GridFold<1>(a, sh, rs, tot) && threadIdx.x == 0) *out = tot[0];
+	YZ_CHUNKS(n)
+	{
+		double a[1] = {0.0};
+		const int i = YZ_CHUNK_ROW;
+		if(i < n)
+		{
+			a[0] = a[0] + x[i] * y[i];
+		}
+		ChunkFold<1>(a, sh, k_, c_, rs);
+	}
+	__syncthreads();
+	if(GridLast<1>(RedChunks(n), sh, rs, tot) && threadIdx.x == 0) *out = tot[0];
 }
-
-#undef YZ_CHUNK_LOOP
 
 //==========================================================================
 //  Fault injection: the switch of the reference's amgcl backend
@@ -682,6 +686,9 @@ void Solver::BuildHierarchy(int coarseEnough)
 	_haveH = true;
 }
 
+//  the blocks of a kernel with a thread a row and no loop over rows
+inline int RowBlocks(int n) { return GridFor(n, kB, 0x7fffffff); }
+
 //  x = V(l) f from a zero guess
 Sten Solver::StenOf(size_t l) const
 {
@@ -702,7 +709,7 @@ void Solver::Cycle(size_t l, const double *f, double *x)
 	if(l + 1 < _nlev)
 	{
 		Level &C = *_levels[l + 1];
-		YZ_LAUNCH(KPreSmoothResidual, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
+		YZ_LAUNCH(KPreSmoothResidual, RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
 		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, x, L.t.get());
 		if(!LaunchCoarse<double>(l))
 		{
@@ -711,13 +718,13 @@ void Solver::Cycle(size_t l, const double *f, double *x)
 			Cycle(l + 1, C.f.get(), C.x.get());
 		}
 		YZ_LAUNCH(KProlong, g, kB, 0, _st, Halt(), n, L.pptr.get(), L.pcol.get(), L.pval.get(), C.x.get(), x, L.xt.get());
-		YZ_LAUNCH(KPostSmooth, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
+		YZ_LAUNCH(KPostSmooth, RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
 		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x, nullptr, 0.0, 0.0);
 	}
 	else
 	{
 		YZ_LAUNCH(KPreSmooth, g, kB, 0, _st, Halt(), n, L.M.get(), f, L.xt.get());
-		YZ_LAUNCH(KPostSmooth, g, kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
+		YZ_LAUNCH(KPostSmooth, RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
 		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x, nullptr, 0.0, 0.0);
 	}
 }
@@ -743,10 +750,10 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 	//  coarser levels (yz_coarse.cuh)
 	if(l == 0 && _nlev > 1 && CoarseCycleOn())
 	{
-		YZ_LAUNCH_PDL((KPreSmoothResidual<float, TF, float>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
+		YZ_LAUNCH_PDL((KPreSmoothResidual<float, TF, float>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
 		          val, L.M32.get(), f, L.x32.get(), L.t32.get());
 		LaunchCoarseCycle();
-		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
+		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
 		          L.M32.get(), f, L.xt32.get(), x, nullptr, 0.0, 0.0);
 		return;
 	}
@@ -771,7 +778,7 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 			if(la > 1) CoarsePreSmooth(la, n, L.ptr.get(), col, val, L.M32.get(), f, L.x32.get(), L.t32.get());
 		}
 		if(la == 1)
-			YZ_LAUNCH_PDL((KPreSmoothResidual<float, TF, float>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
+			YZ_LAUNCH_PDL((KPreSmoothResidual<float, TF, float>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
 			          val, L.M32.get(), f, L.x32.get(), L.t32.get());
 		if(!LaunchCoarse<float>(l))
 		{
@@ -797,22 +804,22 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 			for(int k = 0; k + 1 < K; ++k)
 			{
 				float *xo = (xin == L.xt32.get()) ? L.x32.get() : L.xt32.get();
-				YZ_LAUNCH_PDL((KPostSmooth<float, TF, float, true>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
+				YZ_LAUNCH_PDL((KPostSmooth<float, TF, float, true>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
 				              val, L.M32.get(), f, xin, xo, _lam.get(), SweepRoot(k, K), kSweepRatio);
 				xin = xo;
 			}
 			if(K > 1)
-				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX, true>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
+				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX, true>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
 				              L.M32.get(), f, xin, x, _lam.get(), SweepRoot(K - 1, K), kSweepRatio);
 			else
-				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
+				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
 				              L.M32.get(), f, xin, x, nullptr, 0.0, 0.0);
 		}
 	}
 	else
 	{
 		YZ_LAUNCH_PDL((KPreSmooth<float, TF, float>), g, kB, 0, _st, Halt(), n, L.M32.get(), f, L.xt32.get());
-		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), g, kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val, L.M32.get(), f,
+		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val, L.M32.get(), f,
 		          L.xt32.get(), x, nullptr, 0.0, 0.0);
 	}
 }
@@ -1239,7 +1246,7 @@ void Solver::ApplyPrec(int kind, const double *r, double *z)
 void Solver::EnqueueIteration(int kind)
 {
 	Level &A = *_levels[0];
-	const int n = _n, nb = RedBlocks(n), g = GridFor(n, kB);
+	const int n = _n, nb = RedGrid(n), ns = RedBlocks(n), g = GridFor(n, kB);
 	const int *ptr = A.ptr.get(), *so = _sellOff.get(), *col = _sellCol.get();
 	const double *val = _sellVal.get();
 	//  YZ_PREC_FP32_MATRIX: the SpMVs read the float copy of the values
@@ -1249,15 +1256,15 @@ void Solver::EnqueueIteration(int kind)
 	YZ_LAUNCH_PDL(KPUpdate, g, kB, 0, _st, n, _r.get(), _v.get(), _p.get(), sc);
 	ApplyPrec(kind, _p.get(), _ph.get());
 	if(val32)
-		YZ_LAUNCH_PDL(KSpmvAlpha<float>, nb, kRT, 0, _st, n, ptr, so, _sten, col, val32, _ph.get(), _rh.get(), _v.get(), Red(1), sc);
+		YZ_LAUNCH_PDL(KSpmvAlpha<float>, ns, kRT, 0, _st, n, ptr, so, _sten, col, val32, _ph.get(), _rh.get(), _v.get(), Red(1), sc);
 	else
-		YZ_LAUNCH_PDL(KSpmvAlpha<double>, nb, kRT, 0, _st, n, ptr, so, _sten, col, val, _ph.get(), _rh.get(), _v.get(), Red(1), sc);
+		YZ_LAUNCH_PDL(KSpmvAlpha<double>, ns, kRT, 0, _st, n, ptr, so, _sten, col, val, _ph.get(), _rh.get(), _v.get(), Red(1), sc);
 	YZ_LAUNCH_PDL(KSUpdate, nb, kRT, 0, _st, n, _r.get(), _v.get(), _s.get(), Red(2), sc);
 	ApplyPrec(kind, _s.get(), _sh.get());
 	if(val32)
-		YZ_LAUNCH_PDL(KSpmvOmega<float>, nb, kRT, 0, _st, n, ptr, so, _sten, col, val32, _sh.get(), _s.get(), _t.get(), Red(3), sc);
+		YZ_LAUNCH_PDL(KSpmvOmega<float>, ns, kRT, 0, _st, n, ptr, so, _sten, col, val32, _sh.get(), _s.get(), _t.get(), Red(3), sc);
 	else
-		YZ_LAUNCH_PDL(KSpmvOmega<double>, nb, kRT, 0, _st, n, ptr, so, _sten, col, val, _sh.get(), _s.get(), _t.get(), Red(3), sc);
+		YZ_LAUNCH_PDL(KSpmvOmega<double>, ns, kRT, 0, _st, n, ptr, so, _sten, col, val, _sh.get(), _s.get(), _t.get(), Red(3), sc);
 	YZ_LAUNCH_PDL(KXRUpdate, nb, kRT, 0, _st, n, _ph.get(), _sh.get(), _s.get(), _t.get(), _rh.get(), x, _r.get(),
 	          Red(4), sc);
 }
@@ -1422,13 +1429,13 @@ void Solver::BuildLoopGraph(int kind, LoopGraph &lg)
 bool Solver::BiCGStab(int kind, int maxIter, double tol, int &itOut, double &errOut)
 {
 	Level &A = *_levels[0];
-	const int n = _n, nb = RedBlocks(n), g = GridFor(n, kB);
+	const int n = _n, nb = RedGrid(n), ns = RedBlocks(n), g = GridFor(n, kB);
 	double *b = _b.get(), *x = _x.get();
 	if(_precision == YZ_PREC_FP32_MATRIX)
-		YZ_LAUNCH(KBInit, nb, kRT, 0, _st, n, A.ptr.get(), _sellOff.get(), _sten, _sellCol.get(),
+		YZ_LAUNCH(KBInit, ns, kRT, 0, _st, n, A.ptr.get(), _sellOff.get(), _sten, _sellCol.get(),
 		          (const float *)_sellVal32.get(), b, x, _r.get(), _rh.get(), Red(0), _sc.get());
 	else
-		YZ_LAUNCH(KBInit, nb, kRT, 0, _st, n, A.ptr.get(), _sellOff.get(), _sten, _sellCol.get(), _sellVal.get(), b, x,
+		YZ_LAUNCH(KBInit, ns, kRT, 0, _st, n, A.ptr.get(), _sellOff.get(), _sten, _sellCol.get(), _sellVal.get(), b, x,
 		          _r.get(), _rh.get(), Red(0), _sc.get());
 	YZ_LAUNCH(KCtlStart, 1, 1, 0, _st, _sc.get(), tol, maxIter);
 	YZ_LAUNCH(KZeroIfTiny, g, kB, 0, _st, n, _sc.get(), x);
@@ -1733,7 +1740,7 @@ double DeviceDot(int n, const double *hx, const double *hy)
 	part.reserve((size_t)nb); out.reserve(1); cnt.reserve(1);
 	YZ_CUDA(cudaMemset(cnt.get(), 0, sizeof(unsigned)));
 	RedScratch rs{part.get(), cnt.get(), nb};
-	YZ_LAUNCH(KDot, nb, kRT, 0, 0, n, x.get(), y.get(), rs, out.get());
+	YZ_LAUNCH(KDot, RedGrid(n), kRT, 0, 0, n, x.get(), y.get(), rs, out.get());
 	double h = 0;
 	YZ_CUDA(cudaMemcpy(&h, out.get(), sizeof(double), cudaMemcpyDeviceToHost));
 	return h;
