@@ -113,6 +113,13 @@ def test_gradient_matches_oracle(nx, ny, act):
         assert rel < 5e-2 and cos > 0.995, (a, b, rel, cos)
 
 
+@pytest.mark.parametrize("nx,ny", [(9, 23), (40, 25), (66, 66), (131, 70)])
+def test_gradient_strips_and_groups(nx, ny):
+    """The weight gradient's strips at sizes below one strip, with remainders
+    and with several runs a layer, within the bounds of the test above."""
+    test_gradient_matches_oracle(nx, ny, 0)
+
+
 def _pattern(d):
     return yz.CrsPattern(d["rowptr"], d["col"], d["sorted_col"], d["sorted_src"])
 

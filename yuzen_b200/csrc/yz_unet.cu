@@ -586,87 +586,153 @@ __global__ void KOutMap(int n, int nx, Lv l0, const bf16 *__restrict__ D0, const
 }
 
 //==========================================================================
-//  weight gradients (CUDA cores): block (b, tap) sums
-//  dy[p][n] x[p + dy W + dx][ci] over its pixels [b PB, (b+1) PB) in
-//  pixel order, 32 pixels at a time through shared memory; the partials of
-//  the blocks are summed in block order by KWReduce
+//  Weight gradient.  A block takes the three taps of one row of the stencil
+//  (blockIdx.y) and one run of pixels [b PB, (b+1) PB): partial sums of
+//  dy[p][n] x[p + dy W + dx][ci], summed over the blocks in block order by
+//  KWReduce.
+//
+//  Bound by the FP32 units (6.2 G multiply-adds at 516 x 516: a product of
+//  two bfloat16 is exact in float, so one fused instruction rounds as a
+//  multiply and an add do).  A thread holds a 4 x 4 tile of outputs for the
+//  three taps and walks along a row: the x of two taps stay in its registers
+//  from the pixel before, so two 8-byte reads of shared memory feed 48
+//  multiply-adds.  Where a layer has fewer tiles than the block has threads (16
+//  to 128 of 256) the threads form groups, each with its share of a strip's
+//  pixels, that are summed in group order at the end; a tile a thread alone
+//  left 15 of 16 threads idle at the widest level.  Strips of bfloat16 come in
+//  by 16-byte asynchronous copies, one strip ahead.
 //==========================================================================
-constexpr int kWgJ = 32;
-constexpr int kWgTiles = 2;      // 4 x 4 output tiles per thread (n x cin <= 8192)
+constexpr int kWgT = 256;		// threads
+constexpr int kWgMost = 64;		// pixels a strip
 
-__global__ void __launch_bounds__(256) KWGrad(int H, int W, int cin, int n, int pb, const bf16 *__restrict__ x,
-                                              const bf16 *__restrict__ dy, float *__restrict__ part,
-                                              float *__restrict__ partB)
+__device__ __forceinline__ float4 Bf4(const bf16 *p)
 {
-	__shared__ __align__(16) float sx[kWgJ * 128];
-	__shared__ __align__(16) float sd[kWgJ * 128];
-	const int tap = blockIdx.y;
-	const int ody = tap / 3 - 1, odx = tap % 3 - 1;
+	const uint2 u = *reinterpret_cast<const uint2 *>(p);
+	return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16),
+	                   __uint_as_float(u.y & 0xffff0000u));
+}
+
+__device__ __forceinline__ void CopyStrip16(bf16 *dst, const bf16 *src, bool on)
+{
+	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(on ? 16 : 0) : "memory");
+}
+
+//  S: pixels a strip; dynamic shared memory: two strips of S rows of dy and
+//  S + 2 of x, or the groups' sums (WgSmem)
+__global__ void __launch_bounds__(kWgT, 2) KWGrad(int H, int W, int cin, int n, int pb, int S, const bf16 *__restrict__ x,
+                                                  const bf16 *__restrict__ dy, float *__restrict__ part,
+                                                  float *__restrict__ partB)
+{
+	extern __shared__ __align__(16) unsigned char wsm[];
+	const int t = threadIdx.x, row = blockIdx.y;
 	const int HW = H * W;
-	const int pBeg = blockIdx.x * pb;
-	const int pEnd = min(HW, pBeg + pb);
-	const int outs = n * cin;
-	const int tcs = cin / 4, tiles = (n / 4) * tcs;
-	float acc[kWgTiles][16];
+	const int pBeg = blockIdx.x * pb, pEnd = min(HW, pBeg + pb);
+	const int outs = n * cin, tcs = cin / 4, tiles = (n / 4) * tcs;
+	const int here = min(kWgT, tiles - (int)blockIdx.z * kWgT);	// tiles of this block
+	const int groups = kWgT / here;
+	const int g = t / here, mine = (int)blockIdx.z * kWgT + t - g * here;
+	const int n0 = (mine / tcs) * 4, c0 = (mine - (mine / tcs) * tcs) * 4;
+	const int strip = S * n + (S + 2) * cin;
+	bf16 *buf = reinterpret_cast<bf16 *>(wsm);
+	const int shift = (row - 1) * W - 1;		// x's first pixel of a strip less the strip's
+	auto load = [&](int base, bf16 *to) {
+		const int dv = S * n / 8, xv = (S + 2) * cin / 8;
+		for(int k = t; k < dv; k += kWgT)
+		{
+			const long long e = (long long)base * n + 8LL * k;
+			const bool on = e < (long long)HW * n;
+			CopyStrip16(to + 8 * k, dy + (on ? e : 0), on);
+		}
+		for(int k = t; k < xv; k += kWgT)
+		{
+			const long long e = ((long long)base + shift) * cin + 8LL * k;
+			const bool on = e >= 0 && e < (long long)HW * cin;
+			CopyStrip16(to + S * n + 8 * k, x + (on ? e : 0), on);
+		}
+		asm volatile("cp.async.commit_group;" ::: "memory");
+	};
+	float acc[3][16], accB[4];
 #pragma unroll
-	for(int k = 0; k < kWgTiles; ++k)
+	for(int d = 0; d < 3; ++d)
 #pragma unroll
-		for(int e = 0; e < 16; ++e) acc[k][e] = 0.0f;
-	float accB = 0.0f;
-	for(int base = pBeg; base < pEnd; base += kWgJ)
+		for(int e = 0; e < 16; ++e) acc[d][e] = 0.0f;
+#pragma unroll
+	for(int e = 0; e < 4; ++e) accB[e] = 0.0f;
+	if(pBeg < pEnd) load(pBeg, buf);
+	for(int base = pBeg, k = 0; base < pEnd; base += S, ++k)
 	{
-		for(int idx = threadIdx.x; idx < kWgJ * n; idx += blockDim.x)
-		{
-			const int j = idx / n, c = idx - j * n;
-			const int p = base + j;
-			sd[idx] = (p < pEnd) ? __bfloat162float(dy[(size_t)p * n + c]) : 0.0f;
-		}
-		for(int idx = threadIdx.x; idx < kWgJ * cin; idx += blockDim.x)
-		{
-			const int j = idx / cin, c = idx - j * cin;
-			const int p = base + j;
-			const long long q = (long long)p + (long long)ody * W + odx;
-			sx[idx] = (p < pEnd && q >= 0 && q < HW) ? __bfloat162float(x[(size_t)q * cin + c]) : 0.0f;
-		}
+		bf16 *cur = buf + (k & 1) * strip;
+		if(base + S < pEnd) load(base + S, buf + ((k & 1) ^ 1) * strip);
+		else asm volatile("cp.async.commit_group;" ::: "memory");
+		asm volatile("cp.async.wait_group 1;" ::: "memory");
 		__syncthreads();
-#pragma unroll
-		for(int k = 0; k < kWgTiles; ++k)
+		const int len = min(S, pEnd - base);
+		if(g < groups)
 		{
-			const int t = threadIdx.x + k * blockDim.x;
-			if(t < tiles)
+			const int j0 = g * len / groups, j1 = (g + 1) * len / groups;
+			const bf16 *sd = cur + n0, *sx = cur + S * n + c0;
+			float4 xa = Bf4(sx + j0 * cin), xb = Bf4(sx + (j0 + 1) * cin);
+			for(int j = j0; j < j1; ++j)
 			{
-				const int n0 = (t / tcs) * 4, c0 = (t - (t / tcs) * tcs) * 4;
-				for(int j = 0; j < kWgJ; ++j)
-				{
-					const float4 av = *reinterpret_cast<const float4 *>(&sd[j * n + n0]);
-					const float4 bv = *reinterpret_cast<const float4 *>(&sx[j * cin + c0]);
-					const float ar[4] = {av.x, av.y, av.z, av.w}, br[4] = {bv.x, bv.y, bv.z, bv.w};
+				const float4 av = Bf4(sd + j * n), xc = Bf4(sx + (j + 2) * cin);
+				const float ar[4] = {av.x, av.y, av.z, av.w};
+				const float br[3][4] = {{xa.x, xa.y, xa.z, xa.w}, {xb.x, xb.y, xb.z, xb.w}, {xc.x, xc.y, xc.z, xc.w}};
+#pragma unroll
+				for(int d = 0; d < 3; ++d)
 #pragma unroll
 					for(int u = 0; u < 4; ++u)
 #pragma unroll
-						for(int v = 0; v < 4; ++v) acc[k][u * 4 + v] = acc[k][u * 4 + v] + ar[u] * br[v];
-				}
+						for(int v = 0; v < 4; ++v) acc[d][u * 4 + v] = __fmaf_rn(ar[u], br[d][v], acc[d][u * 4 + v]);
+#pragma unroll
+				for(int u = 0; u < 4; ++u) accB[u] = accB[u] + ar[u];
+				xa = xb; xb = xc;
 			}
 		}
-		if(tap == 0 && threadIdx.x < n)
-			for(int j = 0; j < kWgJ; ++j) accB = accB + sd[j * n + threadIdx.x];
 		__syncthreads();
 	}
+	//  the groups' sums in group order
+	float *red = reinterpret_cast<float *>(wsm);		// [16][kWgT]
+	asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-	for(int k = 0; k < kWgTiles; ++k)
+	for(int d = 0; d < 3; ++d)
 	{
-		const int t = threadIdx.x + k * blockDim.x;
-		if(t < tiles)
+		__syncthreads();
+#pragma unroll
+		for(int e = 0; e < 16; ++e) red[e * kWgT + t] = acc[d][e];
+		__syncthreads();
+		float *dst = part + ((size_t)blockIdx.x * 9 + row * 3 + d) * outs;
+		for(int k = t; k < 16 * here; k += kWgT)
 		{
-			const int n0 = (t / tcs) * 4, c0 = (t - (t / tcs) * tcs) * 4;
-			float *dst = part + ((size_t)blockIdx.x * 9 + tap) * outs;
-#pragma unroll
-			for(int u = 0; u < 4; ++u)
-#pragma unroll
-				for(int v = 0; v < 4; ++v) dst[(n0 + u) * cin + c0 + v] = acc[k][u * 4 + v];
+			const int e = k & 15, m = k >> 4;
+			float s = red[e * kWgT + m];
+			for(int q = 1; q < groups; ++q) s = s + red[e * kWgT + q * here + m];
+			const int tile = (int)blockIdx.z * kWgT + m, tn = tile / tcs;
+			dst[(tn * 4 + (e >> 2)) * cin + (tile - tn * tcs) * 4 + (e & 3)] = s;
 		}
 	}
-	if(tap == 0 && threadIdx.x < n) partB[(size_t)blockIdx.x * n + threadIdx.x] = accB;
+	if(row == 1)
+	{
+		__syncthreads();
+#pragma unroll
+		for(int e = 0; e < 4; ++e) red[e * kWgT + t] = accB[e];
+		__syncthreads();
+		for(int k = t; k < 4 * here; k += kWgT)
+		{
+			const int e = k & 3, m = k >> 2;
+			const int tile = (int)blockIdx.z * kWgT + m, tn = tile / tcs;
+			if(tile != tn * tcs) continue;
+			float s = red[e * kWgT + m];
+			for(int q = 1; q < groups; ++q) s = s + red[e * kWgT + q * here + m];
+			partB[(size_t)blockIdx.x * n + tn * 4 + e] = s;
+		}
+	}
+}
+
+inline size_t WgSmem(int cin, int n, int S)
+{
+	const size_t strips = 2 * sizeof(bf16) * ((size_t)S * n + (size_t)(S + 2) * cin), sums = 16 * kWgT * sizeof(float);
+	return strips > sums ? strips : sums;
 }
 
 //  grad W[n][tap][ci] += sum_b part[b][tap][n][ci]; grad b[n] += sum_b partB[b][n]
@@ -682,6 +748,7 @@ __global__ void KWReduce(int nb, int cin, int n, const float *__restrict__ part,
 			const int tap = k / outs, o = k - tap * outs;
 			const int nn = o / cin, ci = o - nn * cin;
 			float s = 0.0f;
+#pragma unroll 16
 			for(int b = 0; b < nb; ++b) s = s + part[((size_t)b * 9 + tap) * outs + o];
 			const size_t g = wOff + ((size_t)nn * 9 + tap) * cin + ci;
 			grad[g] = grad[g] + s;
@@ -889,15 +956,18 @@ void Learned::WGrad(const ConvLayer &L, const bf16 *x, const bf16 *dy, cudaStrea
 {
 	const Level &lv = _lv[L.level];
 	const int HW = lv.H * lv.W;
-	int pb = (HW + 63) / 64;
-	pb = ((pb + kWgJ - 1) / kWgJ) * kWgJ;
-	if(pb < kWgJ) pb = kWgJ;
-	const int nb = (HW + pb - 1) / pb;
+	//  strips of 64 pixels, 32 where two of them would not fit 48 KB; two
+	//  blocks an SM over the three rows of taps
+	const int S = WgSmem(L.cin, L.cout, kWgMost) <= 48 * 1024 ? kWgMost : kWgMost / 2;
 	const size_t outs = (size_t)L.cout * L.cin;
-	if(outs > (size_t)256 * kWgTiles * 16 || L.cin > 128 || L.cout > 128) throw UsageError("wgrad: layer too wide");
+	const int zs = (int)((outs / 16 + kWgT - 1) / kWgT), want = std::max(1, 2 * 148 / (3 * zs));
+	const int strips = (HW + S - 1) / S, pb = S * ((strips + want - 1) / want);
+	const int nb = (HW + pb - 1) / pb;
+	if(outs > (size_t)kWgT * 32 || L.cin > 128 || L.cout > 128) throw UsageError("wgrad: layer too wide");
 	_part.reserve((size_t)nb * 9 * outs);
 	_partB.reserve((size_t)nb * L.cout);
-	YZ_LAUNCH(KWGrad, dim3(nb, 9), 256, 0, st, lv.H, lv.W, L.cin, L.cout, pb, x, dy, _part.get(), _partB.get());
+	YZ_LAUNCH(KWGrad, dim3(nb, 3, zs), kWgT, WgSmem(L.cin, L.cout, S), st, lv.H, lv.W, L.cin, L.cout, pb, S, x, dy, _part.get(),
+	          _partB.get());
 	YZ_LAUNCH(KWReduce, Blocks((long long)9 * outs + L.cout), 256, 0, st, nb, L.cin, L.cout, _part.get(), _partB.get(),
 	          _grad.get(), L.wOff, L.bOff, _act);
 }
