@@ -573,109 +573,148 @@ __global__ void KGemmFill(int nx, const int *__restrict__ xptr, const int *__res
 }
 
 //--------------------------------------------------------------------------
-//  The same product with one warp per output row: the row's distinct columns
-//  and sums in shared memory (at most CAP), X's row taken entry by entry and
-//  each Y row 32 entries at a time (a Y row holds a column once, so the
-//  lanes of one step never add into the same sum); every sum gets its
-//  contributions in X's row order from 0.0, as the thread-per-row kernels
-//  and the oracle give them.  FILL false: the count of every row (a row
-//  beyond CAP sets *overflow and is done again by KGemmCount<kRowCap>);
-//  FILL true: the row sorted by column into cptr[i]...
+//  The same product with L lanes per output row and at most kGemmCap
+//  distinct columns a row, staged: row i at i kGemmCap, sorted by column, with
+//  its count in cnt[i] (KGemmCompact moves the rows once the counts are
+//  scanned); a row beyond the cap sets *overflow and leaves 0.  ystage: Y's
+//  rows are staged so too, row k with yptr[k] entries.
+//
+//  Bound by latency: a film's row takes 13 short Y rows one after the other,
+//  for every sum gets its contributions in X's row order from 0.0, as the
+//  thread-per-row kernels and the oracle give them (a Y row holds a column
+//  once, so the lanes of one step never add into the same sum).  So four Y
+//  rows are read at once ahead of their sums, and a column's sum is found by a
+//  hash table of 128 places in shared memory (64 columns and one Y row's 32
+//  more always leave it a free place) rather than by a walk over the columns
+//  so far.  The rows of P hold 3 entries on average, so A P gives a row 8
+//  lanes (with 32, instructions for idle lanes bound it); the rows of A P hold
+//  20 to 25, so R (A P) gives 32.  The 18 products of a 512 x 512 step with
+//  rows walked one by one 72 us on average, now 37; 224 x 224 44 and 24.
 //--------------------------------------------------------------------------
-template<int CAP, bool FILL>
-__global__ void __launch_bounds__(256) KGemmWarp(int nx, const int *__restrict__ xptr, const int *__restrict__ xcol,
-                                                 const double *__restrict__ xval, const int *__restrict__ yptr,
-                                                 const int *__restrict__ ycol, const double *__restrict__ yval,
-                                                 int *__restrict__ cnt, const int *__restrict__ cptr,
-                                                 int *__restrict__ ccol, double *__restrict__ cval,
-                                                 int *__restrict__ overflow, bool ystage = false)
+constexpr int kGemmCap = 64, kGemmTab = 128, kGemmThreads = 128;
+
+//  one entry a lane (j < 0: none) into the lanes' row's table; returns the
+//  columns that are new to it (gm: the lanes of the row)
+__device__ __forceinline__ int GemmAdd(int *tcol, double *tval, unsigned gm, int j, double p)
 {
-	constexpr int W = 8;
-	__shared__ int scol[W][CAP];
-	__shared__ double sval[W][FILL ? CAP : 1];
-	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	const unsigned lt = (1u << lane) - 1u;
-	const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
-	for(long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < nx; row += warps)
+	bool fresh = false;
+	if(j >= 0)
 	{
-		const int i = (int)row;
-		int m = 0;
-		bool over = false;
-		const int xe = xptr[i + 1];
-		//  X's row 32 entries at a time: each lane loads one entry and its Y
-		//  row's bounds, which the warp then takes in order by shuffles
-		for(int xb = xptr[i]; xb < xe && !over; xb += 32)
+		unsigned h = ((unsigned)j * 2654435761u) >> 25;
+		for(;;)
 		{
-			const int xk = xb + lane;
+			int have = *(volatile int *)(tcol + h);
+			if(have == -1) have = atomicCAS(tcol + h, -1, j);
+			if(have == -1) { fresh = true; break; }
+			if(have == j) break;
+			h = (h + 1) & (kGemmTab - 1);
+		}
+		tval[h] = (fresh ? 0.0 : tval[h]) + p;
+	}
+	return __popc(__ballot_sync(0xffffffffu, fresh) & gm);
+}
+
+template<int L>
+__global__ void __launch_bounds__(kGemmThreads) KGemmWarp(int nx, const int *__restrict__ xptr, const int *__restrict__ xcol,
+                                                          const double *__restrict__ xval, const int *__restrict__ yptr,
+                                                          const int *__restrict__ ycol, const double *__restrict__ yval,
+                                                          int *__restrict__ cnt, int *__restrict__ ccol,
+                                                          double *__restrict__ cval, int *__restrict__ overflow, bool ystage)
+{
+	constexpr int G = kGemmThreads / L, B = 4;
+	constexpr unsigned all = 0xffffffffu;
+	__shared__ __align__(16) int scol[G][kGemmTab];
+	__shared__ double sval[G][kGemmTab];
+	const int lane = threadIdx.x & 31, l = lane & (L - 1), w = threadIdx.x / L;
+	const unsigned gm = (L == 32 ? all : ((1u << (L & 31)) - 1u)) << (lane & ~(L - 1));
+	const unsigned lt = gm & ((1u << lane) - 1u);
+	int *tc = scol[w];
+	double *tv = sval[w];
+	//  every loop's bounds are the warp's, so that its rows keep together
+	const long long rows = (long long)gridDim.x * G;
+	for(long long r0 = (long long)blockIdx.x * G + (threadIdx.x >> 5) * (32 / L); r0 < nx; r0 += rows)
+	{
+		const long long i = r0 + (lane / L);
+		const bool live = i < nx;
+		const int xs = live ? xptr[i] : 0, xe = live ? xptr[i + 1] : 0;
+		const int xl = __reduce_max_sync(all, xe - xs);
+		int m = 0;
+#pragma unroll
+		for(int q = 4 * l; q < kGemmTab; q += 4 * L) *reinterpret_cast<int4 *>(tc + q) = make_int4(-1, -1, -1, -1);
+		__syncwarp();
+		//  X's row L entries at a time: each lane loads one entry and its Y
+		//  row's bounds, which the row's lanes then take in order by shuffles
+		for(int xo = 0; xo < xl; xo += L)
+		{
+			const int xk = xs + xo + l;
 			const bool av = xk < xe;
 			const int kk = av ? xcol[xk] : 0;
-			const double xvv = (FILL && av) ? xval[xk] : 0.0;
-			//  (ystage: Y's rows staged, row k at k CAP with yptr[k] entries)
+			const double xvv = av ? xval[xk] : 0.0;
 			const int ys = !av ? 0 : ystage ? kk : yptr[kk], yl = !av ? 0 : ystage ? yptr[kk] : yptr[kk + 1] - ys;
-			const int cntx = (xe - xb < 32) ? xe - xb : 32;
-		for(int jx = 0; jx < cntx && !over; ++jx)
-		{
-			const int yr = __shfl_sync(0xffffffffu, ys, jx);
-			const int y1 = __shfl_sync(0xffffffffu, yl, jx);
-			const long long y0 = ystage ? (long long)yr * CAP : (long long)yr;
-			const double xv = __shfl_sync(0xffffffffu, xvv, jx);
-			for(int base = 0; base < y1 && !over; base += 32)
+			const int cntx = min(L, xl - xo);
+			for(int j0 = 0; j0 < cntx; j0 += B)
 			{
-				const int ky = base + lane;
-				const bool active = ky < y1;
-				const int j = active ? ycol[y0 + ky] : -1;
-				int slot = -1;
-				if(active)
-					for(int q = 0; q < m; ++q) if(scol[w][q] == j) { slot = q; break; }
-				const bool need = active && slot < 0;
-				const unsigned mask = __ballot_sync(0xffffffffu, need);
-				const int add = __popc(mask);
-				if(m + add > CAP) { over = true; break; }
-				if(need)
+				int c[B], len[B];
+				double v[B];
+#pragma unroll
+				for(int u = 0; u < B; ++u)
 				{
-					slot = m + __popc(mask & lt);
-					scol[w][slot] = j;
-					if(FILL) sval[w][slot] = 0.0;
+					const int yr = __shfl_sync(all, ys, j0 + u, L);
+					len[u] = __shfl_sync(all, yl, j0 + u, L);
+					const long long y0 = ystage ? (long long)yr * kGemmCap : (long long)yr;
+					const bool on = l < len[u];		// past the row's end: 0
+					c[u] = on ? ycol[y0 + l] : -1;
+					v[u] = on ? yval[y0 + l] : 0.0;
 				}
-				m += add;
-				__syncwarp();
-				if(FILL && active) sval[w][slot] = sval[w][slot] + xv * yval[y0 + ky];
-				__syncwarp();
+#pragma unroll
+				for(int u = 0; u < B; ++u)
+				{
+					const double xv = __shfl_sync(all, xvv, j0 + u, L);
+					m += GemmAdd(tc, tv, gm, m <= kGemmCap ? c[u] : -1, xv * v[u]);
+					__syncwarp();
+					if(!__any_sync(all, len[u] > L)) continue;
+					const int yr = __shfl_sync(all, ys, j0 + u, L), most = __reduce_max_sync(all, len[u]);
+					const long long y0 = (ystage ? (long long)yr * kGemmCap : (long long)yr) + l;
+					for(int k0 = L; k0 < most; k0 += L)
+					{
+						const bool on = k0 + l < len[u] && m <= kGemmCap;
+						m += GemmAdd(tc, tv, gm, on ? ycol[y0 + k0] : -1, on ? xv * yval[y0 + k0] : 0.0);
+						__syncwarp();
+					}
+				}
 			}
 		}
-		}
-		if(!FILL)
+		const bool over = m > kGemmCap;
+		if(live && l == 0)
 		{
-			if(lane == 0)
-			{
-				if(over) { atomicExch(overflow, 1); cnt[i] = 0; }
-				else cnt[i] = m;
-			}
+			if(over) { atomicExch(overflow, 1); cnt[i] = 0; }
+			else cnt[i] = m;
 		}
-		else
+		if(over) m = 0;
+		//  the row's entries together at the front of its table (an entry
+		//  never moves up), then each at its rank among the columns
+		int at = 0;
+		for(int q = 0; q < kGemmTab; q += L)
 		{
-			//  cptr given: the row at its place; else staged at i * CAP with
-			//  its count (KGemmCompact moves it once the counts are scanned)
-			if(!cptr && lane == 0)
-			{
-				if(over) { atomicExch(overflow, 1); cnt[i] = 0; }
-				else cnt[i] = m;
-			}
-			const long long o = cptr ? (long long)cptr[i] : (long long)i * CAP;
-			for(int q = lane; q < m && !over; q += 32)
-			{
-				const int c = scol[w][q];
-				int r = 0;
-				for(int t = 0; t < m; ++t) r += (scol[w][t] < c);
-				ccol[o + r] = c;
-				cval[o + r] = sval[w][q];
-			}
+			const int c = tc[q + l];
+			const double v = tv[q + l];
+			const unsigned mask = __ballot_sync(all, c >= 0);
+			if(c >= 0) { const int to = at + __popc(mask & lt); tc[to] = c; tv[to] = v; }
+			at += __popc(mask & gm);
+			__syncwarp();
+		}
+		const int mw = __reduce_max_sync(all, m);
+		for(int q = l; q < mw; q += L)
+		{
+			const int c = tc[q];
+			int r = 0;
+			for(int t = 0; t < m; ++t) r += tc[t] < c;
+			if(q < m) { ccol[i * kGemmCap + r] = c; cval[i * kGemmCap + r] = tv[q]; }
 		}
 		__syncwarp();
 	}
 }
 
-//  the staged rows (stride CAP) to their places
 template<int CAP>
 __global__ void KGemmCompact(int nx, const int *__restrict__ cptr, const int *__restrict__ tcol,
                              const double *__restrict__ tval, int *__restrict__ ccol, double *__restrict__ cval)

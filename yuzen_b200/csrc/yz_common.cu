@@ -102,6 +102,7 @@ namespace {
 thread_local std::string t_lastError;
 constexpr int kScanBlock = 1024;
 
+//  a block's 1,024 counts (exclusive); a single block writes the total too
 __global__ void ScanBlocks(const int *__restrict__ in, int *__restrict__ out, int n, int *__restrict__ blockSums)
 {
 	__shared__ int warpSums[kScanBlock / 32];
@@ -129,7 +130,11 @@ __global__ void ScanBlocks(const int *__restrict__ in, int *__restrict__ out, in
 	__syncthreads();
 	const int incl = v + (warp > 0 ? warpSums[warp - 1] : 0);
 	if(i < n) out[i] = incl - ((i < n) ? in[i] : 0);	// exclusive within the block
-	if(threadIdx.x == kScanBlock - 1) blockSums[blockIdx.x] = incl;
+	if(threadIdx.x == kScanBlock - 1)
+	{
+		blockSums[blockIdx.x] = incl;
+		if(gridDim.x == 1) out[n] = incl;
+	}
 }
 
 //  one block scans the block sums in tiles of 1024 (exclusive), total at end
@@ -179,6 +184,23 @@ __global__ void ScanAdd(int *out, int n, const int *blockSums, const int *total)
 	if(i < n) out[i] += blockSums[blockIdx.x];
 	if(i == 0) out[n] = *total;
 }
+
+//  ScanAdd on the blocks' own sums: every block adds up those before it, which
+//  spares a launch of one block between the two
+__global__ void ScanAddSums(int *out, int n, const int *blockSums)
+{
+	__shared__ int warpSums[kScanBlock / 32];
+	const int i = blockIdx.x * kScanBlock + threadIdx.x;
+	int s = 0;
+	for(int k = threadIdx.x; k < (int)blockIdx.x; k += kScanBlock) s += blockSums[k];
+	for(int off = 16; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+	if((threadIdx.x & 31) == 0) warpSums[threadIdx.x >> 5] = s;
+	__syncthreads();
+	s = warpSums[threadIdx.x & 31];
+	for(int off = 16; off >= 1; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+	if(i < n) out[i] += s;
+	if(blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) out[n] = s + blockSums[blockIdx.x];
+}
 } // namespace
 
 void SetLastError(const std::string &m) { t_lastError = m; }
@@ -196,6 +218,15 @@ void ScanExclusive(const int *in, int *out, int n, int *scratch, cudaStream_t st
 	}
 	int *sums = scratch, *total = scratch + nb;
 	YZ_LAUNCH(ScanBlocks, nb, kScanBlock, 0, st, in, out, n, sums);
+	if(nb == 1) return;
+	//  A set-up scans five times a level and a launch is 2.4 us whatever it
+	//  does; past 2,048 blocks (2 M rows) the sums that every block adds up
+	//  would be more to read than the counts
+	if(nb <= 2048)
+	{
+		YZ_LAUNCH(ScanAddSums, nb, kScanBlock, 0, st, out, n, sums);
+		return;
+	}
 	YZ_LAUNCH(ScanSums, 1, kScanBlock, 0, st, sums, nb, total);
 	YZ_LAUNCH(ScanAdd, nb, kScanBlock, 0, st, out, n, sums, total);
 }

@@ -651,11 +651,11 @@ void Solver::BuildHierarchy(int coarseEnough)
 		//  AP staged, 64 places a row, then A_c = R (AP) from the staged rows
 		_apCnt.reserve((size_t)n); _apCol.reserve((size_t)n * 64); _apVal.reserve((size_t)n * 64);
 		_gtCol.reserve((size_t)nc * 64); _gtVal.reserve((size_t)nc * 64);
-		YZ_LAUNCH((KGemmWarp<64, true>), GridFor((long long)n * 32, 256, 148 * 64), 256, 0, _st, n, L.ptr.get(), L.col.get(),
-		          L.val.get(), L.pptr.get(), L.pcol.get(), L.pval.get(), _apCnt.get(), nullptr, _apCol.get(), _apVal.get(),
+		YZ_LAUNCH(KGemmWarp<8>, GridFor((long long)n * 8, kGemmThreads, 148 * 64), kGemmThreads, 0, _st, n, L.ptr.get(), L.col.get(),
+		          L.val.get(), L.pptr.get(), L.pcol.get(), L.pval.get(), _apCnt.get(), _apCol.get(), _apVal.get(),
 		          overflow, false);
-		YZ_LAUNCH((KGemmWarp<64, true>), GridFor((long long)nc * 32, 256, 148 * 64), 256, 0, _st, nc, L.rptr.get(),
-		          L.rcol.get(), L.rval.get(), _apCnt.get(), _apCol.get(), _apVal.get(), _cnt.get(), nullptr, _gtCol.get(),
+		YZ_LAUNCH(KGemmWarp<32>, GridFor((long long)nc * 32, kGemmThreads, 148 * 64), kGemmThreads, 0, _st, nc, L.rptr.get(),
+		          L.rcol.get(), L.rval.get(), _apCnt.get(), _apCol.get(), _apVal.get(), _cnt.get(), _gtCol.get(),
 		          _gtVal.get(), overflow, true);
 		C.ptr.reserve((size_t)nc + 1);
 		ScanExclusive(_cnt.get(), C.ptr.get(), nc, _scan.get(), _st);
