@@ -163,6 +163,7 @@ __global__ void KScaleGather(int n, const int *__restrict__ rowptr, const int *_
 __global__ void KDiag(int n, const int *__restrict__ ptr, const int *__restrict__ col,
                       const double *__restrict__ val, double *__restrict__ dia)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		double d = 0.0;
@@ -178,6 +179,7 @@ __global__ void KStrength(int n, const int *__restrict__ ptr, const int *__restr
                           const double *__restrict__ val, const double *__restrict__ dia, double eps2,
                           unsigned char *__restrict__ strong, int *__restrict__ cnt)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		const double e = eps2 * dia[i];
@@ -200,6 +202,7 @@ __global__ void KStrength(int n, const int *__restrict__ ptr, const int *__restr
 __global__ void KFillIn(int n, const int *__restrict__ ptr, const int *__restrict__ col,
                         const unsigned char *__restrict__ strong, int *__restrict__ fill, int *__restrict__ nbr)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		int out = 0;
@@ -220,6 +223,7 @@ __global__ void KFillIn(int n, const int *__restrict__ ptr, const int *__restric
 __global__ void KMisInit(int n, const int *__restrict__ nptr, int *__restrict__ state, unsigned char *__restrict__ iso,
                          unsigned long long *__restrict__ T0, int *__restrict__ undecided)
 {
+	PdlEntry();
 	int cnt = 0;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
@@ -253,6 +257,7 @@ __global__ void KMisMax(int n, const int *__restrict__ nptr, const int *__restri
                         const unsigned long long *__restrict__ Tin, unsigned long long *__restrict__ Tout,
                         const int *__restrict__ undecided, int *zero)
 {
+	PdlEntry();
 	if(blockIdx.x == 0 && threadIdx.x == 0) *zero = 0;
 	if(*undecided == 0) return;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -263,6 +268,7 @@ __global__ void KMisUpdate(int n, const int *__restrict__ nptr, const int *__res
                            const unsigned long long *__restrict__ T1, int *__restrict__ state,
                            unsigned long long *__restrict__ T0, const int *__restrict__ undecided, int *__restrict__ next)
 {
+	PdlEntry();
 	if(*undecided == 0) return;
 	int cnt = 0;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -283,6 +289,7 @@ __global__ void KMisUpdate(int n, const int *__restrict__ nptr, const int *__res
 
 __global__ void KRootFlags(int n, const int *__restrict__ state, int *__restrict__ flag)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) flag[i] = state[i] == kIn ? 1 : 0;
 }
 
@@ -290,6 +297,7 @@ __global__ void KAssignFirst(int n, const int *__restrict__ nptr, const int *__r
                              const int *__restrict__ state, const unsigned char *__restrict__ iso,
                              const int *__restrict__ rootId, int *__restrict__ first)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		if(state[i] == kIn) { first[i] = rootId[i]; continue; }
@@ -304,6 +312,7 @@ __global__ void KAssignFirst(int n, const int *__restrict__ nptr, const int *__r
 __global__ void KAssignSecond(int n, const int *__restrict__ nptr, const int *__restrict__ nbr,
                               const unsigned char *__restrict__ iso, const int *__restrict__ first, int *__restrict__ agg)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		if(first[i] >= 0 || iso[i]) { agg[i] = first[i]; continue; }
@@ -324,6 +333,7 @@ __global__ void KSpai0(int n, const int *__restrict__ ptr, const int *__restrict
                        const double *__restrict__ val, double *__restrict__ M, float *__restrict__ M32,
                        unsigned long long *lam)
 {
+	PdlEntry();
 	unsigned long long most = 0, least = ~0ull;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
@@ -384,6 +394,7 @@ __global__ void KPCount(int n, const int *__restrict__ ptr, const int *__restric
                         const unsigned char *__restrict__ strong, const int *__restrict__ agg,
                         int *__restrict__ cnt, int *__restrict__ overflow)
 {
+	PdlEntry();
 	int lc[CAP];
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
@@ -408,6 +419,7 @@ __global__ void KPFill(int n, const int *__restrict__ ptr, const int *__restrict
                        const int *__restrict__ agg, const int *__restrict__ pptr,
                        int *__restrict__ pcol, double *__restrict__ pval)
 {
+	PdlEntry();
 	const double omega = 2.0 / 3.0;
 	int lc[CAP];
 	double lv[CAP];
@@ -446,6 +458,7 @@ __global__ void KPFill(int n, const int *__restrict__ ptr, const int *__restrict
 //  R = P^T: counts per column, atomic fill, then each row sorted by fine row
 __global__ void KColCount(const int *__restrict__ total, const int *__restrict__ pcol, int *__restrict__ cnt)
 {
+	PdlEntry();
 	const int nnz = *total;
 	for(int k = blockIdx.x * blockDim.x + threadIdx.x; k < nnz; k += gridDim.x * blockDim.x) atomicAdd(&cnt[pcol[k]], 1);
 }
@@ -454,6 +467,7 @@ __global__ void KTransposeFill(int n, const int *__restrict__ pptr, const int *_
                                const double *__restrict__ pval, int *__restrict__ fill,
                                int *__restrict__ rcol, double *__restrict__ rval)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 		for(int k = pptr[i]; k < pptr[i + 1]; ++k)
 		{
@@ -468,6 +482,7 @@ __global__ void KTransposeFill(int n, const int *__restrict__ pptr, const int *_
 __global__ void __launch_bounds__(256) KRowSort(int n, const int *__restrict__ ptr, int *__restrict__ col,
                                                 double *__restrict__ val)
 {
+	PdlEntry();
 	constexpr int L = 64, W = 8;
 	__shared__ int sc[W][L];
 	__shared__ double sv[W][L];
@@ -621,6 +636,7 @@ __global__ void __launch_bounds__(kGemmThreads) KGemmWarp(int nx, const int *__r
                                                           int *__restrict__ cnt, int *__restrict__ ccol,
                                                           double *__restrict__ cval, int *__restrict__ overflow, bool ystage)
 {
+	PdlEntry();
 	constexpr int G = kGemmThreads / L, B = 4;
 	constexpr unsigned all = 0xffffffffu;
 	__shared__ __align__(16) int scol[G][kGemmTab];
@@ -719,6 +735,7 @@ template<int CAP>
 __global__ void KGemmCompact(int nx, const int *__restrict__ cptr, const int *__restrict__ tcol,
                              const double *__restrict__ tval, int *__restrict__ ccol, double *__restrict__ cval)
 {
+	PdlEntry();
 	for(long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < (long long)nx * CAP;
 	    e += (long long)gridDim.x * blockDim.x)
 	{

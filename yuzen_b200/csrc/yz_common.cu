@@ -105,6 +105,7 @@ constexpr int kScanBlock = 1024;
 //  a block's 1,024 counts (exclusive); a single block writes the total too
 __global__ void ScanBlocks(const int *__restrict__ in, int *__restrict__ out, int n, int *__restrict__ blockSums)
 {
+	PdlEntry();
 	__shared__ int warpSums[kScanBlock / 32];
 	const int i = blockIdx.x * kScanBlock + threadIdx.x;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -140,6 +141,7 @@ __global__ void ScanBlocks(const int *__restrict__ in, int *__restrict__ out, in
 //  one block scans the block sums in tiles of 1024 (exclusive), total at end
 __global__ void ScanSums(int *blockSums, int nb, int *total)
 {
+	PdlEntry();
 	__shared__ int warpSums[kScanBlock / 32];
 	__shared__ int carry;
 	if(threadIdx.x == 0) carry = 0;
@@ -180,6 +182,7 @@ __global__ void ScanSums(int *blockSums, int nb, int *total)
 
 __global__ void ScanAdd(int *out, int n, const int *blockSums, const int *total)
 {
+	PdlEntry();
 	const int i = blockIdx.x * kScanBlock + threadIdx.x;
 	if(i < n) out[i] += blockSums[blockIdx.x];
 	if(i == 0) out[n] = *total;
@@ -189,6 +192,7 @@ __global__ void ScanAdd(int *out, int n, const int *blockSums, const int *total)
 //  spares a launch of one block between the two
 __global__ void ScanAddSums(int *out, int n, const int *blockSums)
 {
+	PdlEntry();
 	__shared__ int warpSums[kScanBlock / 32];
 	const int i = blockIdx.x * kScanBlock + threadIdx.x;
 	int s = 0;
@@ -217,18 +221,18 @@ void ScanExclusive(const int *in, int *out, int n, int *scratch, cudaStream_t st
 		return;
 	}
 	int *sums = scratch, *total = scratch + nb;
-	YZ_LAUNCH(ScanBlocks, nb, kScanBlock, 0, st, in, out, n, sums);
+	YZ_LAUNCH_PDL(ScanBlocks, nb, kScanBlock, 0, st, in, out, n, sums);
 	if(nb == 1) return;
 	//  A set-up scans five times a level and a launch is 2.4 us whatever it
 	//  does; past 2,048 blocks (2 M rows) the sums that every block adds up
 	//  would be more to read than the counts
 	if(nb <= 2048)
 	{
-		YZ_LAUNCH(ScanAddSums, nb, kScanBlock, 0, st, out, n, sums);
+		YZ_LAUNCH_PDL(ScanAddSums, nb, kScanBlock, 0, st, out, n, sums);
 		return;
 	}
-	YZ_LAUNCH(ScanSums, 1, kScanBlock, 0, st, sums, nb, total);
-	YZ_LAUNCH(ScanAdd, nb, kScanBlock, 0, st, out, n, sums, total);
+	YZ_LAUNCH_PDL(ScanSums, 1, kScanBlock, 0, st, sums, nb, total);
+	YZ_LAUNCH_PDL(ScanAdd, nb, kScanBlock, 0, st, out, n, sums, total);
 }
 
 } // namespace yz

@@ -61,6 +61,7 @@ inline int GjPanelWidth(int n) { return n <= 2 * kGjThreads ? 16 : 8; }
 __global__ void KGjInit(int n, const int *__restrict__ ptr, const int *__restrict__ col,
                         const double *__restrict__ val, double *__restrict__ Mc, int *__restrict__ orig)
 {
+	PdlEntry();
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
 	{
 		orig[i] = i;
@@ -335,6 +336,7 @@ __global__ void __launch_bounds__(kGjThreads, 1) KGjStep(int n, double *__restri
                                                          double *__restrict__ Fn, int kN, int bN,
                                                          int *__restrict__ orig)
 {
+	PdlEntry();
 	__shared__ __align__(16) double rowK[kGjMaxB][kGjCols];
 	__shared__ double Fs[kGjMaxB][kGjRows];  // the multipliers of the listed rows
 	__shared__ unsigned touched[96];         // a bit a row: listed (n <= 3000)
@@ -371,6 +373,7 @@ __global__ void __launch_bounds__(kGjThreads, 1) KGjStep(int n, double *__restri
 __global__ void __launch_bounds__(256) KGjExtract(int n, const double *__restrict__ Mc, const int *__restrict__ orig,
                                                   double *__restrict__ inv)
 {
+	PdlEntry();
 	__shared__ double tile[32][33];
 	const int nt = (n + 31) / 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 	for(int q = blockIdx.x; q < nt * nt; q += gridDim.x)
