@@ -35,6 +35,13 @@ bool PdlOn()
 	return on;
 }
 
+bool ChainOn()
+{
+	static const char *env = std::getenv("YZ_PDL");
+	static const bool on = !env || env[0] != '0';
+	return on;
+}
+
 bool TimingActive() { return g_timeOn.load(std::memory_order_acquire); }
 
 void TimeBegin(cudaStream_t st)
@@ -221,18 +228,18 @@ void ScanExclusive(const int *in, int *out, int n, int *scratch, cudaStream_t st
 		return;
 	}
 	int *sums = scratch, *total = scratch + nb;
-	YZ_LAUNCH_PDL(ScanBlocks, nb, kScanBlock, 0, st, in, out, n, sums);
+	YZ_LAUNCH_CHAIN(ScanBlocks, nb, kScanBlock, 0, st, in, out, n, sums);
 	if(nb == 1) return;
 	//  A set-up scans five times a level and a launch is 2.4 us whatever it
 	//  does; past 2,048 blocks (2 M rows) the sums that every block adds up
 	//  would be more to read than the counts
 	if(nb <= 2048)
 	{
-		YZ_LAUNCH_PDL(ScanAddSums, nb, kScanBlock, 0, st, out, n, sums);
+		YZ_LAUNCH_CHAIN(ScanAddSums, nb, kScanBlock, 0, st, out, n, sums);
 		return;
 	}
-	YZ_LAUNCH_PDL(ScanSums, 1, kScanBlock, 0, st, sums, nb, total);
-	YZ_LAUNCH_PDL(ScanAdd, nb, kScanBlock, 0, st, out, n, sums, total);
+	YZ_LAUNCH_CHAIN(ScanSums, 1, kScanBlock, 0, st, sums, nb, total);
+	YZ_LAUNCH_CHAIN(ScanAdd, nb, kScanBlock, 0, st, out, n, sums, total);
 }
 
 } // namespace yz

@@ -74,15 +74,21 @@ void TimeDropLast(long long k);   // forget the last k of them
 		::yz::Check(cudaGetLastError(), #kernel);                                 \
 	} while(0)
 
-//  Programmatic dependent launch for the chains of short kernels in the
-//  BiCGStab loop and the V-cycle: a kernel launched by YZ_LAUNCH_PDL may be
-//  scheduled while the kernel before it on the stream drains.  Such a kernel
-//  begins with PdlEntry(): griddepcontrol.wait holds every thread until the
-//  kernels it depends on have completed and their memory is visible (so its
-//  reads and writes are those of a plain launch), then launch_dependents lets
-//  the next kernel be scheduled.  Without the launch attribute both are no-ops.
-//  YZ_PDL=0 in the environment launches these kernels plainly.
+//  Programmatic dependent launch for chains of short kernels: a kernel
+//  launched by YZ_LAUNCH_CHAIN (the AMG set-up) or YZ_LAUNCH_PDL (the BiCGStab
+//  loop and the V-cycle) may be scheduled while the kernel before it on the
+//  stream drains.  Such a kernel begins with PdlEntry(): griddepcontrol.wait
+//  holds every thread until the kernels it depends on have completed and their
+//  memory is visible (so its reads and writes are those of a plain launch),
+//  then launch_dependents lets the next kernel be scheduled.  Without the
+//  launch attribute both are no-ops.
+//  The set-up's 70 kernels a hierarchy are queued on the stream, where it pays:
+//  64^2 1.81 -> 1.42 ms, 224^2 3.95 -> 3.23, 301^2 4.4 -> 3.6, and the direct
+//  level's 242 launches at 1,936 rows 7.7 -> 7.2.  The loop's lie in a graph,
+//  where it does not (a 512^2 solve in 64 bits 7.7 without, 7.9 with), so there it
+//  is off.  YZ_PDL=0 in the environment turns it off for both, YZ_PDL=1 on.
 bool PdlOn();
+bool ChainOn();
 __device__ __forceinline__ void PdlEntry()
 {
 #if defined(__CUDA_ARCH__)
@@ -90,11 +96,13 @@ __device__ __forceinline__ void PdlEntry()
 	asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #endif
 }
-#define YZ_LAUNCH_PDL(kernel, grid, block, smem, strm, ...)                     \
+#define YZ_LAUNCH_PDL(...) YZ_LAUNCH_PDL_IF(::yz::PdlOn(), __VA_ARGS__)
+#define YZ_LAUNCH_CHAIN(...) YZ_LAUNCH_PDL_IF(::yz::ChainOn(), __VA_ARGS__)
+#define YZ_LAUNCH_PDL_IF(pdl, kernel, grid, block, smem, strm, ...)             \
 	do {                                                                          \
 		const bool yzTimed_ = ::yz::TimedKernel(#kernel);                         \
 		if(yzTimed_) ::yz::TimeBegin(strm);                                     \
-		if(::yz::PdlOn())                                                         \
+		if(pdl)                                                                 \
 		{                                                                         \
 			cudaLaunchConfig_t yzCfg_ = {};                                       \
 			yzCfg_.gridDim = dim3(grid);                                          \

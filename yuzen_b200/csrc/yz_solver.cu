@@ -517,13 +517,13 @@ int Solver::WideGemm(int nx, const int *xptr, const int *xcol, const double *xva
 
 template<int CAP> void Solver::CountP(Level &L, int *overflow)
 {
-	YZ_LAUNCH_PDL((KPCount<CAP>), GridFor(L.n, kB), kB, 0, _st, L.n, L.ptr.get(), L.col.get(), _strong.get(), L.agg.get(), _cnt.get(),
+	YZ_LAUNCH_CHAIN((KPCount<CAP>), GridFor(L.n, kB), kB, 0, _st, L.n, L.ptr.get(), L.col.get(), _strong.get(), L.agg.get(), _cnt.get(),
 	          overflow);
 }
 
 template<int CAP> void Solver::FillP(Level &L)
 {
-	YZ_LAUNCH_PDL((KPFill<CAP>), GridFor(L.n, kB), kB, 0, _st, L.n, L.ptr.get(), L.col.get(), L.val.get(), _strong.get(), L.agg.get(),
+	YZ_LAUNCH_CHAIN((KPFill<CAP>), GridFor(L.n, kB), kB, 0, _st, L.n, L.ptr.get(), L.col.get(), L.val.get(), _strong.get(), L.agg.get(),
 	          L.pptr.get(), L.pcol.get(), L.pval.get());
 }
 
@@ -540,7 +540,7 @@ void Solver::DirectInverse(Level &L)
 	_gjOrig.reserve((size_t)n);
 	double *Mc = _gj[0].get(), *F[2] = {_gj[1].get(), _gj[1].get() + (size_t)B * n};
 	YZ_CUDA(cudaMemsetAsync(Mc, 0, (size_t)n * n * sizeof(double), _st));
-	YZ_LAUNCH_PDL(KGjInit, GridFor(n, kB), kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), Mc, _gjOrig.get());
+	YZ_LAUNCH_CHAIN(KGjInit, GridFor(n, kB), kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), Mc, _gjOrig.get());
 	auto kernel = n <= 256 ? KGjStep<16, 1, 2, 1> : n <= 512 ? KGjStep<16, 1, 1, 1> : n <= 1024 ? KGjStep<16, 2, 1, 1> :
 	              n <= 2048 ? KGjStep<8, 4, 1, 2> : KGjStep<8, 6, 1, 2>;
 	const int tiles = std::min((n + kGjCols - 1) / kGjCols, 147);
@@ -549,12 +549,12 @@ void Solver::DirectInverse(Level &L)
 		//  panel q (from k - B on) applied, the next one (from k on) factored
 		const GjPanel *prev = q < 0 ? nullptr : _gjPan.get() + (q & 1);
 		const int bNext = std::max(0, std::min(B, n - k));
-		YZ_LAUNCH_PDL(kernel, q < 0 ? 1 : 1 + tiles, kGjThreads, 0, _st, n, Mc, prev, F[q & 1], _gjPan.get() + ((q + 1) & 1),
+		YZ_LAUNCH_CHAIN(kernel, q < 0 ? 1 : 1 + tiles, kGjThreads, 0, _st, n, Mc, prev, F[q & 1], _gjPan.get() + ((q + 1) & 1),
 		          F[(q + 1) & 1], k, bNext, _gjOrig.get());
 		k += B;
 	}
 	L.inv.reserve((size_t)n * n);
-	YZ_LAUNCH_PDL(KGjExtract, std::min(148 * 8, ((n + 31) / 32) * ((n + 31) / 32)), 256, 0, _st, n, Mc, _gjOrig.get(), L.inv.get());
+	YZ_LAUNCH_CHAIN(KGjExtract, std::min(148 * 8, ((n + 31) / 32) * ((n + 31) / 32)), 256, 0, _st, n, Mc, _gjOrig.get(), L.inv.get());
 }
 
 //--------------------------------------------------------------------------
@@ -584,40 +584,40 @@ void Solver::BuildHierarchy(int coarseEnough)
 		}
 		//  strength, and the list of every row's strong neighbours
 		_strong.reserve((size_t)nnz); _icol.reserve(2 * (size_t)nnz);
-		YZ_LAUNCH_PDL(KDiag, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _dia.get());
+		YZ_LAUNCH_CHAIN(KDiag, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _dia.get());
 		YZ_CUDA(cudaMemsetAsync(_icnt.get(), 0, ((size_t)n + 1) * sizeof(int), _st));
-		YZ_LAUNCH_PDL(KStrength, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _dia.get(), eps * eps,
+		YZ_LAUNCH_CHAIN(KStrength, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), _dia.get(), eps * eps,
 		          _strong.get(), _icnt.get());
 		eps *= 0.5;
 		ScanExclusive(_icnt.get(), _iptr.get(), n, _scan.get(), _st);
 		YZ_CUDA(cudaMemcpyAsync(_ifill.get(), _iptr.get(), (size_t)n * sizeof(int), cudaMemcpyDeviceToDevice, _st));
-		YZ_LAUNCH_PDL(KFillIn, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _ifill.get(), _icol.get());
+		YZ_LAUNCH_CHAIN(KFillIn, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), _strong.get(), _ifill.get(), _icol.get());
 		//  MIS-2 (at most 64 rounds, as the oracle): eight rounds, nearly always
 		//  enough, are queued before the host reads how many rows are left
 		int *undec = _flags.get() + 4;		// two counters, by round parity
 		YZ_CUDA(cudaMemsetAsync(undec, 0, 2 * sizeof(int), _st));
-		YZ_LAUNCH_PDL(KMisInit, g, kB, 0, _st, n, _iptr.get(), _state.get(), _iso.get(), _T0.get(), undec);
+		YZ_LAUNCH_CHAIN(KMisInit, g, kB, 0, _st, n, _iptr.get(), _state.get(), _iso.get(), _T0.get(), undec);
 		int nc = 0;
 		for(int round = 0; round < 64;)
 		{
 			for(int end = round + (round ? 4 : 8); round < end; ++round)
 			{
 				int *u = undec + (round & 1), *un = undec + ((round + 1) & 1);
-				YZ_LAUNCH_PDL(KMisMax, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _T0.get(), _T1.get(), u, un);
-				YZ_LAUNCH_PDL(KMisUpdate, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _T1.get(), _state.get(), _T0.get(), u, un);
+				YZ_LAUNCH_CHAIN(KMisMax, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _T0.get(), _T1.get(), u, un);
+				YZ_LAUNCH_CHAIN(KMisUpdate, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _T1.get(), _state.get(), _T0.get(), u, un);
 			}
 			//  the aggregates' roots, with the count of rows left
-			YZ_LAUNCH_PDL(KRootFlags, g, kB, 0, _st, n, _state.get(), _flag.get());
+			YZ_LAUNCH_CHAIN(KRootFlags, g, kB, 0, _st, n, _state.get(), _flag.get());
 			int left = 0;
 			nc = ScanCounts(_flag.get(), _rootId.get(), n, undec + (round & 1), &left);
 			if(left == 0) break;
 		}
-		YZ_LAUNCH_PDL(KAssignFirst, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _state.get(), _iso.get(), _rootId.get(),
+		YZ_LAUNCH_CHAIN(KAssignFirst, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _state.get(), _iso.get(), _rootId.get(),
 		          _first.get());
-		YZ_LAUNCH_PDL(KAssignSecond, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _iso.get(), _first.get(), L.agg.get());
+		YZ_LAUNCH_CHAIN(KAssignSecond, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _iso.get(), _first.get(), L.agg.get());
 		unsigned long long *lam = l == 0 && _precision != YZ_PREC_FP64 ? reinterpret_cast<unsigned long long *>(_lam.get()) : nullptr;
 		if(lam) ClearBounds();
-		YZ_LAUNCH_PDL(KSpai0, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), L.M.get(), nullptr, lam);
+		YZ_LAUNCH_CHAIN(KSpai0, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), L.M.get(), nullptr, lam);
 		L.nc = nc;
 		if(nc == 0) break;		// nothing to coarsen: this level is smoothed only
 		if(_levels.size() <= l + 1) _levels.emplace_back(new Level());
@@ -641,20 +641,20 @@ void Solver::BuildHierarchy(int coarseEnough)
 		//  R = P^T
 		L.rptr.reserve((size_t)nc + 1); L.rcol.reserve((size_t)nnz); L.rval.reserve((size_t)nnz);
 		YZ_CUDA(cudaMemsetAsync(_cnt.get(), 0, ((size_t)nc + 1) * sizeof(int), _st));
-		YZ_LAUNCH_PDL(KColCount, gz, kB, 0, _st, L.pptr.get() + n, L.pcol.get(), _cnt.get());
+		YZ_LAUNCH_CHAIN(KColCount, gz, kB, 0, _st, L.pptr.get() + n, L.pcol.get(), _cnt.get());
 		ScanExclusive(_cnt.get(), L.rptr.get(), nc, _scan.get(), _st);
 		YZ_CUDA(cudaMemcpyAsync(_ifill.get(), L.rptr.get(), (size_t)nc * sizeof(int), cudaMemcpyDeviceToDevice, _st));
-		YZ_LAUNCH_PDL(KTransposeFill, g, kB, 0, _st, n, L.pptr.get(), L.pcol.get(), L.pval.get(), _ifill.get(),
+		YZ_LAUNCH_CHAIN(KTransposeFill, g, kB, 0, _st, n, L.pptr.get(), L.pcol.get(), L.pval.get(), _ifill.get(),
 		          L.rcol.get(), L.rval.get());
-		YZ_LAUNCH_PDL(KRowSort, GridFor((long long)nc * 32, 256, 148 * 64), 256, 0, _st, nc, L.rptr.get(), L.rcol.get(),
+		YZ_LAUNCH_CHAIN(KRowSort, GridFor((long long)nc * 32, 256, 148 * 64), 256, 0, _st, nc, L.rptr.get(), L.rcol.get(),
 		          L.rval.get());
 		//  AP staged, 64 places a row, then A_c = R (AP) from the staged rows
 		_apCnt.reserve((size_t)n); _apCol.reserve((size_t)n * 64); _apVal.reserve((size_t)n * 64);
 		_gtCol.reserve((size_t)nc * 64); _gtVal.reserve((size_t)nc * 64);
-		YZ_LAUNCH_PDL((KGemmWarp<8>), GridFor((long long)n * 8, kGemmThreads, 148 * 64), kGemmThreads, 0, _st, n, L.ptr.get(), L.col.get(),
+		YZ_LAUNCH_CHAIN((KGemmWarp<8>), GridFor((long long)n * 8, kGemmThreads, 148 * 64), kGemmThreads, 0, _st, n, L.ptr.get(), L.col.get(),
 		          L.val.get(), L.pptr.get(), L.pcol.get(), L.pval.get(), _apCnt.get(), _apCol.get(), _apVal.get(),
 		          overflow, false);
-		YZ_LAUNCH_PDL((KGemmWarp<32>), GridFor((long long)nc * 32, kGemmThreads, 148 * 64), kGemmThreads, 0, _st, nc, L.rptr.get(),
+		YZ_LAUNCH_CHAIN((KGemmWarp<32>), GridFor((long long)nc * 32, kGemmThreads, 148 * 64), kGemmThreads, 0, _st, nc, L.rptr.get(),
 		          L.rcol.get(), L.rval.get(), _apCnt.get(), _apCol.get(), _apVal.get(), _cnt.get(), _gtCol.get(),
 		          _gtVal.get(), overflow, true);
 		C.ptr.reserve((size_t)nc + 1);
@@ -670,7 +670,7 @@ void Solver::BuildHierarchy(int coarseEnough)
 		{
 			C.most = 64;
 			C.col.reserve((size_t)C.nnz); C.val.reserve((size_t)C.nnz);
-			YZ_LAUNCH_PDL((KGemmCompact<64>), GridFor((long long)nc * 64, 256, 148 * 64), 256, 0, _st, nc, C.ptr.get(),
+			YZ_LAUNCH_CHAIN((KGemmCompact<64>), GridFor((long long)nc * 64, 256, 148 * 64), 256, 0, _st, nc, C.ptr.get(),
 			          _gtCol.get(), _gtVal.get(), C.col.get(), C.val.get());
 		}
 		else
@@ -1511,7 +1511,7 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 	if(set.conc && set.precondition == 2 && _offSpai.Try())
 	{
 		YZ_PROF("lin.fallback.conc", _st);
-		YZ_LAUNCH_PDL(KSpai0, g, kB, 0, _st, n, L0.ptr.get(), L0.col.get(), L0.val.get(), _m.get(), nullptr, nullptr);
+		YZ_LAUNCH_CHAIN(KSpai0, g, kB, 0, _st, n, L0.ptr.get(), L0.col.get(), L0.val.get(), _m.get(), nullptr, nullptr);
 		if(!BiCGStab(kPrecDiag, tryIter, set.epsilon, it, err)) err = 1e300;
 		if(err <= set.epsilon) { done = true; _offSpai.Converged(); }
 		else
@@ -1567,7 +1567,7 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 		{
 			{
 				YZ_PROF("lin.precond", _st);
-				YZ_LAUNCH_PDL(KDiag, g, kB, 0, _st, n, L0.ptr.get(), L0.col.get(), L0.val.get(), _dia.get());
+				YZ_LAUNCH_CHAIN(KDiag, g, kB, 0, _st, n, L0.ptr.get(), L0.col.get(), L0.val.get(), _dia.get());
 				YZ_LAUNCH(KDampedJacobi, g, kB, 0, _st, n, _dia.get(), _m.get());
 			}
 			YZ_PROF("lin.iterate", _st);
@@ -1595,7 +1595,7 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 						{
 							unsigned long long *lam = fp32 ? reinterpret_cast<unsigned long long *>(_lam.get()) : nullptr;
 							if(lam) ClearBounds();
-							YZ_LAUNCH_PDL(KSpai0, g, kB, 0, _st, n, F.ptr.get(), F.col.get(), F.val.get(), F.M.get(),
+							YZ_LAUNCH_CHAIN(KSpai0, g, kB, 0, _st, n, F.ptr.get(), F.col.get(), F.val.get(), F.M.get(),
 							          fp32 ? F.M32.get() : nullptr, lam);
 						}
 						++_sinceBuild;
