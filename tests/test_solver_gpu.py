@@ -521,3 +521,31 @@ def test_wide_rows_bitwise(width):
     assert_same(g[:4], o.solve(d))
     assert g[0] == 0
     _levels_equal(g[4].levels(), o.levels())
+
+
+@pytest.mark.parametrize("served", [0, 8])
+def test_reused_hierarchy_is_stale_only_when_old(served):
+    """A solve that takes far more iterations than the set-up's first makes
+    the next one set up afresh once the hierarchy has served eight solves;
+    before that its count becomes the reference and the hierarchy stays."""
+    d = _systems.film_system(100, seed=4)
+    easy, hard = dict(d, epsilon=1e-1), dict(d, epsilon=1e-12)
+    e, h = (_oracle.OracleSolver().solve(q) for q in (easy, hard))
+    assert e[0] == 0 and h[0] == 0 and h[1] > e[1] + max(4, e[1] // 2) + 2
+    be = yz.B200Backend()
+    be.SetAmgReuse(64)
+
+    pat = yz.CrsPattern(d["rowptr"], d["col"], d["sorted_col"], d["sorted_src"])
+
+    def launches(q):
+        l0, x = be.launches(), np.zeros(d["n"])
+        s = yz.LinearSolverSettings(int(q["precondition"]), bool(q["scaling"]), int(q["max_iteration"]),
+                                    float(q["epsilon"]), bool(q["conc"]))
+        assert be.Solve(s, pat, q["values"], q["rhs"], x)[0] == 0
+        return be.launches() - l0
+
+    launches(easy)
+    for _ in range(served):
+        launches(easy)
+    first, then = launches(hard), launches(hard)
+    assert (then > first) if served else (then == first), (first, then)
