@@ -88,7 +88,10 @@ int yz_solver_solve(yz_solver* s, const yz_settings* set, const double* values,
 int yz_solver_solve_device(yz_solver* s, const yz_settings* set, const double* d_values,
                            const double* d_rhs, double* d_x, int* iter, double* resid);
 
-/* Preconditioner arithmetic (YZ_PREC_*), from the next solve on. */
+/* Preconditioner arithmetic (YZ_PREC_*), from the next solve on.  In the FP32
+ * forms a run that breaks down, or ends no nearer than it began, on a new
+ * set-up's Chebyshev sweeps is repeated from the initial guess on sweeps of
+ * weight 1 (iter counts both runs), unless that has not helped of late. */
 int yz_solver_set_precision(yz_solver* s, int precision);
 
 /* AMG hierarchy reuse.  0 (the default, the reference's way): a new SA-AMG
@@ -330,8 +333,9 @@ int yz_step_set_graph_loop(yz_step* st, int on);
  * each (-1: the library's default, level 2 or YZ_FUSE_FROM; 0: none),
  * coarse_lanes the lanes a row of the coarse levels' kernels (0: by the
  * level's mean row length; 1, 2, 4 or 8), fine_sweeps the post-smoothing
- * sweeps at the finest level, a Chebyshev iteration (0: the default, 8 or
- * YZ_FINE_SWEEPS; 1 to 8).
+ * sweeps at the finest level (0: the default, 8 or YZ_FINE_SWEEPS; 1 to 8),
+ * a Chebyshev iteration where that damps the set-up's system better than
+ * sweeps of weight 1 (tried at every set-up).
  * The launch shapes change the preconditioner by float rounding only, the
  * sweeps change it (a better one); the FP64 cycle, the reference's, is not
  * affected.  yuzen_b200.autotune picks them per instance size. */

@@ -86,3 +86,24 @@ def poisson1d(n: int) -> dict:
     return {"n": n, "nnz": int(rowptr[-1]), "rowptr": rowptr, "col": col, "sorted_col": scol,
             "sorted_src": ssrc, "values": val, "rhs": rhs, "x0": np.zeros(n), "precondition": 2,
             "scaling": 1, "max_iteration": 10 * n, "epsilon": 1e-13, "conc": 0, "exact": x_exact, "dx": dx}
+
+
+def upwind_system(N: int, courant: float, stiff: float, order: int = 1, seed: int = 3) -> dict:
+    """film_system's grid, pattern and ghost rows with I + upwind advection
+    (Courant numbers `courant` and half of it along x and y, first or second
+    order) + stiff times the biharmonic stencil on the interior rows: a
+    spectrum with imaginary parts as large as its real ones where `stiff` is
+    small."""
+    d = film_system(N, seed=seed)
+    nx = N + 4
+    jj, ii = np.divmod(np.arange(d["n"]), nx)
+    base = d["rowptr"][:-1][(ii >= 2) & (ii < nx - 2) & (jj >= 2) & (jj < nx - 2)]
+    row = stiff * _BIH
+    row[0] += 1.0
+    for c, near, far in ((courant, 1, 5), (0.5 * courant, 3, 7)):
+        row[0] += c if order == 1 else 1.5 * c
+        row[near] -= c if order == 1 else 2.0 * c
+        row[far] += 0.0 if order == 1 else 0.5 * c
+    d["values"] = d["values"].copy()
+    d["values"][base[:, None] + np.arange(13)] = row
+    return dict(d, scaling=0, epsilon=1e-10, max_iteration=500)

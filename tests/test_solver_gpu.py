@@ -549,3 +549,36 @@ def test_reused_hierarchy_is_stale_only_when_old(served):
         launches(easy)
     first, then = launches(hard), launches(hard)
     assert (then > first) if served else (then == first), (first, then)
+
+
+@pytest.mark.parametrize("precision", [yz.PREC_FP32_CYCLE, yz.PREC_FP32_MATRIX])
+@pytest.mark.parametrize("courant,stiff,order", [(3, 0.0, 1), (5, 0.0, 1), (5, 0.3, 1), (2, 0.3, 2)])
+@pytest.mark.parametrize("N", [60, 124])
+def test_advection_dominated_systems_in_fp32(N, courant, stiff, order, precision):
+    """Upwind systems whose eigenvalues have large imaginary parts, in one
+    cluster (60) and as separate launches (124): the FP32 forms converge, in
+    no more iterations than with the reference's one sweep in the same
+    arithmetic."""
+    d = _systems.upwind_system(N, courant, stiff, order)
+    runs = []
+    for sweeps in (0, 1):
+        be = yz.B200Backend()
+        be.SetPrecision(precision)
+        be.SetTuning(-1, 0, sweeps)
+        runs.append(gpu_solve(d, be))
+    g, one = runs
+    assert one[0] == 0 and g[0] == 0 and g[2] <= 1e-10 and g[1] <= one[1], (g[:3], one[:3])
+    rounding = 0.0 if precision == yz.PREC_FP32_CYCLE else 4.0 * 2.0 ** -24 * _abs_product(d, g[3])
+    assert _true_residual(d, g[3]) <= 2e-10 + rounding
+
+
+def test_hopeless_run_is_repeated_on_plain_sweeps_once():
+    """A run of the FP32 cycle that ends no nearer than it began is repeated
+    with sweeps of weight 1 (its iterations count too); where that does not
+    help either, the next such run is not repeated."""
+    d = _systems.film_system(124, seed=124, stiff=1e4)
+    d["epsilon"], d["max_iteration"] = 1e-10, 3     # (restated in 64 bits: the residual 3.8 times the first)
+    be = yz.B200Backend()
+    be.SetPrecision(yz.PREC_FP32_CYCLE)
+    first, then = gpu_solve(d, be), gpu_solve(d, be)
+    assert first[0] == then[0] == 1 and first[1] == 6 and then[1] == 3, (first[:3], then[:3])

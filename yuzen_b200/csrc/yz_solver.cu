@@ -217,9 +217,10 @@ __global__ void KCtlInit(Scal *sc, double eps, int maxIter)
 //  before its loop): |b| < 2 eps_machine gives x = 0 and no iteration; else
 //  eps = tol |b|, and the loop runs while the start residual is above it and
 //  an iteration is allowed
-__global__ void KCtlStart(Scal *sc, double tol, int maxIter)
+__global__ void KCtlStart(Scal *sc, double tol, int maxIter, const double *lam)
 {
 	sc->maxIter = maxIter; sc->it = 0; sc->bodies = 0;
+	sc->res0 = sc->res; sc->plain = lam[2] != 0.0;
 	const double normB = sc->normb;
 	if(normB < 2.0 * 2.220446049250313e-16) { sc->state = kTiny; return; }
 	const double eps = tol * normB;
@@ -335,7 +336,8 @@ Solver::Solver(int device, cudaStream_t stream) : _device(device)
 	YZ_CUDA(cudaEventCreateWithFlags(&_evRing[0], cudaEventDisableTiming));
 	YZ_CUDA(cudaEventCreateWithFlags(&_evRing[1], cudaEventDisableTiming));
 	_sc.reserve(1);
-	_lam.reserve(2);
+	_lam.reserve(3);
+	YZ_CUDA(cudaMemsetAsync(_lam.get(), 0, 3 * sizeof(double), _st));
 	_counters.reserve(16);
 	YZ_CUDA(cudaMemsetAsync(_counters.get(), 0, 16 * sizeof(unsigned), _st));
 	_flags.reserve(8);
@@ -355,6 +357,10 @@ Solver::~Solver()
 	cudaEventDestroy(_evRing[0]); cudaEventDestroy(_evRing[1]);
 	cudaEventDestroy(_ev0); cudaEventDestroy(_ev1); cudaEventDestroy(_ev2);
 	FreeLoopGraph(_loop[0]); FreeLoopGraph(_loop[1]); FreeLoopGraph(_loop[2]);
+	FreeLoopGraph(_probeGraph);
+	if(_stProbe) { cudaStreamSynchronize(_stProbe); cudaStreamDestroy(_stProbe); }
+	if(_evSpai) cudaEventDestroy(_evSpai);
+	if(_evProbe) cudaEventDestroy(_evProbe);
 	if(_ownStream) cudaStreamDestroy(_st);
 }
 
@@ -570,6 +576,12 @@ void Solver::BuildHierarchy(int coarseEnough)
 	++_epochH;
 	++_rebuilds;
 	_nlev = 1;
+	//  what follows on the stream waits for the trial, however this ends
+	struct Join
+	{
+		cudaStream_t st; const cudaEvent_t &done; bool running;
+		~Join() { if(running) cudaStreamWaitEvent(st, done, 0); }
+	} probe{_st, _evProbe, false};
 	double eps = 0.08;
 	for(size_t l = 0;; ++l)
 	{
@@ -619,10 +631,19 @@ void Solver::BuildHierarchy(int coarseEnough)
 		          _first.get());
 		YZ_LAUNCH_CHAIN(KAssignSecond, g, kB, 0, _st, n, _iptr.get(), _icol.get(), _iso.get(), _first.get(), L.agg.get());
 		unsigned long long *lam = l == 0 && _precision != YZ_PREC_FP64 ? reinterpret_cast<unsigned long long *>(_lam.get()) : nullptr;
-		if(lam) ClearBounds();
-		YZ_LAUNCH_CHAIN(KSpai0, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), L.M.get(), nullptr, lam);
+		if(lam)
+		{
+			ClearBounds();
+			L.M32.reserve((size_t)n);
+		}
+		YZ_LAUNCH_CHAIN(KSpai0, g, kB, 0, _st, n, L.ptr.get(), L.col.get(), L.val.get(), L.M.get(), lam ? L.M32.get() : nullptr, lam);
 		L.nc = nc;
 		if(nc == 0) break;		// nothing to coarsen: this level is smoothed only
+		if(lam && FineSweeps() > 1)
+		{
+			if(_offCheb.Try()) { ProbeSweeps(); probe.running = true; }
+			else YZ_LAUNCH(KFill, 1, 1, 0, _st, 1, 1.0, _lam.get() + 2);
+		}
 		if(_levels.size() <= l + 1) _levels.emplace_back(new Level());
 		_nlev = l + 2;
 		Level &C = *_levels[l + 1];
@@ -930,6 +951,69 @@ void Solver::ClearBounds()
 	YZ_CUDA(cudaMemsetAsync(_lam.get() + 1, 0xff, sizeof(double), _st));
 }
 
+//  The trial of the finest level's sweeps (KProbeStart), two rounds of either
+//  kind, in the vectors that hold M p and M s during a run.  On a stream of
+//  its own beside the rest of the set-up, which leaves most of the chip idle,
+//  and as one graph, for the host's time to queue 18 launches is the set-up's:
+//  a 301^2 set-up of 1.9 ms took 88 us more with them in line, 55 us more
+//  queued beside it, and 4 us more so.
+void Solver::ProbeSweeps()
+{
+	if(!_stProbe)
+	{
+		YZ_CUDA(cudaEventCreateWithFlags(&_evSpai, cudaEventDisableTiming));
+		YZ_CUDA(cudaEventCreateWithFlags(&_evProbe, cudaEventDisableTiming));
+		YZ_CUDA(cudaStreamCreateWithFlags(&_stProbe, cudaStreamNonBlocking));
+	}
+	LoopGraph &pg = _probeGraph;
+	const bool direct = TimingActive();		// a timed kernel's events are not recorded in a graph
+	if(!direct && (pg.exec == nullptr || pg.key != _epoch))
+	{
+		FreeLoopGraph(pg);
+		const long long l0 = t_launches;
+		YZ_CUDA(cudaStreamBeginCapture(_stProbe, cudaStreamCaptureModeThreadLocal));
+		try
+		{
+			EnqueueProbe();
+		}
+		catch(...)
+		{
+			cudaGraph_t dummy = nullptr;
+			if(cudaStreamEndCapture(_stProbe, &dummy) == cudaSuccess && dummy) cudaGraphDestroy(dummy);
+			throw;
+		}
+		YZ_CUDA(cudaStreamEndCapture(_stProbe, &pg.graph));
+		pg.perBody = t_launches - l0;
+		CountLaunches(-pg.perBody);
+		YZ_CUDA(cudaGraphInstantiate(&pg.exec, pg.graph, 0));
+		pg.key = _epoch;
+	}
+	YZ_CUDA(cudaEventRecord(_evSpai, _st));
+	YZ_CUDA(cudaStreamWaitEvent(_stProbe, _evSpai, 0));
+	if(direct) EnqueueProbe();
+	else
+	{
+		YZ_CUDA(cudaGraphLaunch(pg.exec, _stProbe));
+		CountLaunches(pg.perBody);
+	}
+	YZ_CUDA(cudaEventRecord(_evProbe, _stProbe));
+}
+
+void Solver::EnqueueProbe()
+{
+	Level &L = *_levels[0];
+	const int n = L.n, K = FineSweeps();
+	float2 *x = reinterpret_cast<float2 *>(_ph.get()), *y = reinterpret_cast<float2 *>(_sh.get());
+	YZ_LAUNCH(KProbeStart, GridFor(n, kB), kB, 0, _stProbe, n, x, _lam.get());
+	for(int k = 0; k < 2 * K; ++k)
+	{
+		YZ_LAUNCH(KProbeSweep, RowBlocks(n), kB, 0, _stProbe, n, L.ptr.get(), _sellOff.get(), _sten, _sellCol.get(),
+		          _sellVal32.get(), L.M32.get(), x, y, _lam.get(), SweepRoot(k % K, K), kSweepRatio);
+		std::swap(x, y);
+	}
+	YZ_LAUNCH(KProbeJudge, RedBlocks(n), kRT, 0, _stProbe, n, x, Red(5), _lam.get());
+}
+
 int Solver::FineSweeps() const
 {
 	static const char *env = std::getenv("YZ_FINE_SWEEPS");
@@ -945,6 +1029,7 @@ void Solver::SetTuning(int fuseFrom, int coarseLanes, int fineSweeps)
 		throw UsageError("set_tuning: coarse_lanes must be 0 (by row length), 1, 2, 4 or 8");
 	if(fuseFrom != _fuseFrom || coarseLanes != _coarseLanes || fineSweeps != _fineSweeps)
 		++_epoch;   // the loop graph holds the old shapes
+	if(fineSweeps != _fineSweeps) _stale = true;   // the kind of sweeps was chosen for the old number
 	_fuseFrom = fuseFrom;
 	_coarseLanes = coarseLanes;
 	_fineSweeps = fineSweeps;
@@ -1440,7 +1525,7 @@ bool Solver::BiCGStab(int kind, int maxIter, double tol, int &itOut, double &err
 	else
 		YZ_LAUNCH(KBInit, ns, kRT, 0, _st, n, A.ptr.get(), _sellOff.get(), _sten, _sellCol.get(), _sellVal.get(), b, x,
 		          _r.get(), _rh.get(), Red(0), _sc.get());
-	YZ_LAUNCH(KCtlStart, 1, 1, 0, _st, _sc.get(), tol, maxIter);
+	YZ_LAUNCH(KCtlStart, 1, 1, 0, _st, _sc.get(), tol, maxIter, _lam.get());
 	YZ_LAUNCH(KZeroIfTiny, g, kB, 0, _st, n, _sc.get(), x);
 	RunIterations(kind);
 	const Scal &h = *_hsc;
@@ -1618,8 +1703,28 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 					YZ_PROF("lin.iterate", _st);
 					broke = !BiCGStab(kPrecAmg, set.max_iteration, set.epsilon, it, err);
 				}
+				//  A run that broke down on Chebyshev sweeps, or ended no nearer than it
+				//  began, is repeated from the caller's guess on sweeps of weight 1.
+				//  If that mends it the next set-ups take those sweeps; if not, the
+				//  next such runs are not repeated.
+				const bool failed = broke || (it > 0 && !(_hsc->res < _hsc->res0));
+				if(failed && !reuse && fp32 && !_levels[0]->direct && _nlev > 1 && FineSweeps() > 1 && !_hsc->plain &&
+				   _offPlain.Try())
+				{
+					itTried += broke ? 0 : it;
+					YZ_CUDA(cudaMemcpyAsync(_x.get(), _x0.get(), (size_t)n * sizeof(double), cudaMemcpyDeviceToDevice, _st));
+					YZ_LAUNCH(KFill, 1, 1, 0, _st, 1, 1.0, _lam.get() + 2);
+					broke = !BiCGStab(kPrecAmg, set.max_iteration, set.epsilon, it, err);
+					if(!broke && err <= set.epsilon) { _offPlain.Converged(); _offCheb.Failed(); }
+					else _offPlain.Failed();
+				}
 				if(!broke && !set.conc && err <= set.epsilon) _amgIters = it;
-				if(!reuse) { _freshIters = it; break; }
+				if(!reuse)
+				{
+					if(!_hsc->plain && !broke && err <= set.epsilon) _offCheb.Converged();
+					_freshIters = it;
+					break;
+				}
 				if(broke || !(err <= set.epsilon))
 				{
 					//  the old hierarchy failed where a new one may not: set up

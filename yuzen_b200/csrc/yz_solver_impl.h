@@ -19,9 +19,11 @@ struct Scal
 {
 	double normb, res, rho, rhoPrev, alpha, omega;
 	double eps;              // tol * |b|
+	double res0;             // the start residual
 	int it, maxIter;         // iterations done, the cap
 	int state;               // 0 running; see KState
 	int bodies;              // iterations queued and run (the graph's loop count)
+	int plain;               // the cycle's finest level takes sweeps of weight 1 (KProbeJudge)
 };
 
 //  the state word of a BiCGStab run on the device
@@ -129,6 +131,8 @@ private:
 	static double SweepRoot(int k, int K);
 	static constexpr double kSweepRatio = 1.0 / 20.0;
 	void ClearBounds();
+	void ProbeSweeps();
+	void EnqueueProbe();
 	//  launch shapes asked for (SetTuning) on the FP32 cycle's separate
 	//  launches: the one-cluster forms stand back
 	bool ShapesSet() const { return _precision != YZ_PREC_FP64 && (_fuseFrom >= 0 || _coarseLanes > 0); }
@@ -164,6 +168,8 @@ private:
 	cudaStream_t _st = nullptr;
 	bool _ownStream = true;
 	cudaEvent_t _ev0 = nullptr, _ev1 = nullptr, _ev2 = nullptr;
+	cudaStream_t _stProbe = nullptr;    // ProbeSweeps, beside the set-up's stream
+	cudaEvent_t _evSpai = nullptr, _evProbe = nullptr;
 	int _n = 0, _nnz = 0;
 	std::vector<int> _hptr, _hcol;
 	DBuf<int> _ssrc;
@@ -184,7 +190,9 @@ private:
 	int _partBlocks = 1;
 	DBuf<unsigned> _counters;
 	DBuf<Scal> _sc;
-	DBuf<double> _lam;          // bounds of the spectrum of M A at the finest level (the FP32 cycle's; KSpai0)
+	//  the FP32 cycle's finest level: bounds of the spectrum of M A (KSpai0), and
+	//  not 0 where its sweeps have weight 1 (KProbeJudge)
+	DBuf<double> _lam;
 	Scal *_hsc = nullptr;
 	int *_hint = nullptr;      // pinned: totals and flags read back together
 	Scal *_hring = nullptr;    // pinned: the state after the last two iterations
@@ -203,6 +211,7 @@ private:
 	DBuf<GjPanel> _gjPan;
 	DBuf<int> _gjOrig;
 	TryBackoff _offSpai;
+	TryBackoff _offCheb, _offPlain;     // Chebyshev sweeps; the repeat of a failed run on plain ones
 	//  hierarchy reuse (0: a new set-up every solve, the reference's way)
 	int _amgReuse = 0, _sinceBuild = 0, _freshIters = 0, _rebuilds = 0;
 	bool _stale = false;
@@ -215,6 +224,7 @@ private:
 	//  by the level's mean row length)
 	int _fuseFrom = -1, _coarseLanes = 0, _fineSweeps = 0;
 	LoopGraph _loop[3];
+	LoopGraph _probeGraph;        // ProbeSweeps
 	bool _graphLoop = true;       // the loop as a CUDA graph (else from the stream)
 	//  Solve's tail, queued behind a graph run: x into the caller's dX
 	double *_tailDst = nullptr;
