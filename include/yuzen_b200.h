@@ -102,7 +102,8 @@ int yz_solver_set_precision(yz_solver* s, int precision);
  * graph.  A solve on a reused hierarchy that fails is repeated on a new
  * set-up; one that takes clearly more iterations than the set-up's first
  * solve (more than max(4, half) again) makes the next solve set up afresh, or,
- * within eight solves of a set-up, is what later solves are held to instead.
+ * within eight solves of a set-up and with no more than twice the iterations a
+ * digit of the residual (and 4), is what later solves are held to instead.
  * The Krylov solve stays FP64 to the same tolerance. */
 int yz_solver_set_amg_reuse(yz_solver* s, int max_solves);
 

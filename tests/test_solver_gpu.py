@@ -582,3 +582,31 @@ def test_hopeless_run_is_repeated_on_plain_sweeps_once():
     be.SetPrecision(yz.PREC_FP32_CYCLE)
     first, then = gpu_solve(d, be), gpu_solve(d, be)
     assert first[0] == then[0] == 1 and first[1] == 6 and then[1] == 3, (first[:3], then[:3])
+
+
+def _striped_system(N: int, kx: float, ky: float) -> dict:
+    """film_system's grid and pattern with I - kx d2/dx2 - ky d2/dy2 on the
+    interior rows: the aggregates of its hierarchy lie along the larger one."""
+    d = _systems.film_system(N, seed=4)
+    nx = N + 4
+    jj, ii = np.divmod(np.arange(d["n"]), nx)
+    base = d["rowptr"][:-1][(ii >= 2) & (ii < nx - 2) & (jj >= 2) & (jj < nx - 2)]
+    row = np.zeros(13)
+    row[:5] = 1.0 + 2.0 * (kx + ky), -kx, -kx, -ky, -ky
+    d["values"] = d["values"].copy()
+    d["values"][base[:, None] + np.arange(13)] = row
+    return dict(d, scaling=0, epsilon=1e-12, max_iteration=500)
+
+
+def test_young_hierarchy_of_another_system_is_stale():
+    """A film that turns into another one on the second solve of a set-up: its
+    solve takes far more iterations a digit than the set-up's did, so the
+    next one sets up afresh, however young the hierarchy is."""
+    x, y = _striped_system(100, 10.0, 0.1), _striped_system(100, 0.1, 10.0)
+    fresh = [_oracle.OracleSolver().solve(q)[1] for q in (x, y)]
+    be = yz.B200Backend()
+    be.SetAmgReuse(64)
+    pat = yz.CrsPattern(x["rowptr"], x["col"], x["sorted_col"], x["sorted_src"])
+    s = yz.LinearSolverSettings(2, False, 500, 1e-12, False)
+    its = [be.Solve(s, pat, q["values"], q["rhs"], np.zeros(q["n"]))[1] for q in (x, x, y, y, y)]
+    assert its[0] == fresh[0] and its[2] > 3 * fresh[1] and its[3] == fresh[1] and its[4] <= fresh[1] + 4, (its, fresh)

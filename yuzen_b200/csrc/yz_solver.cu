@@ -1557,6 +1557,13 @@ double Solver::BreakdownResidual()
 	return (bb > 0.0) ? std::sqrt(rr / bb) : std::sqrt(rr);
 }
 
+//  the decimal digits by which a run lowered its residual, within 1 to 16
+static double Digits(const Scal &s)
+{
+	const double d = s.res > 0.0 ? std::log10(s.res0 / s.res) : 16.0;
+	return d >= 1.0 ? std::min(d, 16.0) : 1.0;
+}
+
 int Solver::Solve(const yz_settings &set, const double *dValues, const double *dRhs, double *dX, int &iterOut, double &residOut)
 {
 	if(_n <= 0) throw UsageError("solve: set_pattern first");
@@ -1723,6 +1730,7 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 				{
 					if(!_hsc->plain && !broke && err <= set.epsilon) _offCheb.Converged();
 					_freshIters = it;
+					_freshRate = it / Digits(*_hsc);
 					break;
 				}
 				if(broke || !(err <= set.epsilon))
@@ -1735,14 +1743,18 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 					continue;
 				}
 				//  A count that grows on a hierarchy of a few solves is the
-				//  system's, not the hierarchy's age: it becomes what later ones
-				//  are held to.  (The first solve of a time step takes more
-				//  iterations than the later ones, so a set-up at one of those
-				//  was called stale by the next step's first: a set-up, 1.2 of
-				//  7.3 ms, in every step of the 512^2 film from its fifth on.)
+				//  system's and not the hierarchy's age while the residual falls
+				//  about as fast as in the set-up's own solve: it becomes what
+				//  later ones are held to.  (The first solve of a time step asks
+				//  for the fewest digits, so a set-up at one of those was called
+				//  stale by the step's last: a set-up, 1.2 of 7.3 ms, in every step
+				//  of the 512^2 film from its fifth on.  Its solves take 2 to 8
+				//  iterations, 0.42 to 0.61 a digit; over nine films the count
+				//  varies by a factor of 5, the iterations a digit by 2.6 where
+				//  the set-up's solve took one, by 2.1 at most where it took more.)
 				if(it > _freshIters + std::max(4, _freshIters / 2))
 				{
-					if(_sinceBuild < kYoungSolves) _freshIters = it;
+					if(_sinceBuild < kYoungSolves && it <= 4 + 2.0 * _freshRate * Digits(*_hsc)) _freshIters = it;
 					else _stale = true;
 				}
 				break;

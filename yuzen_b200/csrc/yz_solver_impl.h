@@ -214,6 +214,7 @@ private:
 	TryBackoff _offCheb, _offPlain;     // Chebyshev sweeps; the repeat of a failed run on plain ones
 	//  hierarchy reuse (0: a new set-up every solve, the reference's way)
 	int _amgReuse = 0, _sinceBuild = 0, _freshIters = 0, _rebuilds = 0;
+	double _freshRate = 0.0;      // iterations a digit of the set-up's own solve
 	bool _stale = false;
 	int _hPrec = YZ_PREC_FP64;    // the precision the present hierarchy was set up in
 	//  bumped whenever a pointer or size a loop graph holds may change: the
