@@ -610,3 +610,40 @@ def test_young_hierarchy_of_another_system_is_stale():
     s = yz.LinearSolverSettings(2, False, 500, 1e-12, False)
     its = [be.Solve(s, pat, q["values"], q["rhs"], np.zeros(q["n"]))[1] for q in (x, x, y, y, y)]
     assert its[0] == fresh[0] and its[2] > 3 * fresh[1] and its[3] == fresh[1] and its[4] <= fresh[1] + 4, (its, fresh)
+
+
+def _weak_system(n: int) -> dict:
+    """A band of n rows without a strong connection: nothing is aggregated,
+    so the cycle smooths its finest level only."""
+    rng = np.random.default_rng(n)
+    rows = [[i] + [j for j in (i - 70, i - 1, i + 1, i + 70) if 0 <= j < n] for i in range(n)]
+    rowptr = np.zeros(n + 1, np.int32)
+    rowptr[1:] = np.cumsum([len(r) for r in rows])
+    col = np.array([c for r in rows for c in r], np.int32)
+    val = rng.uniform(-0.07, 0.07, col.size)
+    val[rowptr[:-1]] = 1.0
+    scol, ssrc = _systems.sorted_mirror(rowptr, col)
+    return {"n": n, "nnz": col.size, "rowptr": rowptr, "col": col, "sorted_col": scol, "sorted_src": ssrc,
+            "values": val, "rhs": rng.standard_normal(n), "x0": np.zeros(n), "precondition": 2, "scaling": 0,
+            "max_iteration": 100, "epsilon": 1e-11, "conc": 0}
+
+
+@pytest.mark.parametrize("n", [3001, 4096, 12001, 20481])
+def test_nothing_to_coarsen(n):
+    """A finest level with nothing coarser: the FP64 solve is the oracle's to
+    the bit, and the FP32 cycle's is the same in one cluster and as separate
+    launches (a launch shape asked for), below and above the sizes that take
+    the one and the other."""
+    d = _weak_system(n)
+    o = _oracle.OracleSolver()
+    r = o.solve(d)
+    assert len(o.levels()) == 1 and not o.levels()[0]["direct"]
+    assert_same(gpu_solve(d)[:4], r)
+    runs = []
+    for shape in ((-1, 0, 0), (0, 0, 0)):
+        be = yz.B200Backend()
+        be.SetPrecision(yz.PREC_FP32_CYCLE)
+        be.SetTuning(*shape)
+        runs.append(gpu_solve(d, be))
+    assert runs[0][0] == 0
+    assert_same(runs[0][:4], runs[1][:4])

@@ -1244,7 +1244,8 @@ template<class T> bool Solver::FillPlan(ClPlan<T> &P, size_t l0) const
 {
 	if(_nlev - l0 > (size_t)kClMaxLevels) return false;
 	P.count = (int)(_nlev - l0);
-	P.sweeps = std::is_same<T, float>::value ? FineSweeps() : 1;
+	//  as Cycle32: a finest level with nothing coarser takes one plain sweep
+	P.sweeps = std::is_same<T, float>::value && _nlev > 1 ? FineSweeps() : 1;
 	P.lam = _lam.get();
 	P.ratio = kSweepRatio;
 	for(int k = 0; k < P.sweeps; ++k) P.root[k] = SweepRoot(k, P.sweeps);
