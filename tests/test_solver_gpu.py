@@ -647,3 +647,40 @@ def test_nothing_to_coarsen(n):
         runs.append(gpu_solve(d, be))
     assert runs[0][0] == 0
     assert_same(runs[0][:4], runs[1][:4])
+
+
+@pytest.mark.parametrize("n", [1936, 2047, 2048, 2049, 2560, 2561, 3000])
+def test_direct_level_bitwise_large(n):
+    """The direct level's inverse with four and six rows a thread: around
+    2,048 rows, where the last of a thread's rows starts, and at its limit."""
+    d = _swapping_system(n, n)
+    assert_same(gpu_solve(d)[:4], _oracle.OracleSolver().solve(d))
+
+
+@pytest.mark.parametrize("n", [33, 300, 1100, 2100])
+@pytest.mark.parametrize("kind", ["zero row", "zero column", "twin rows", "loose block", "inf", "nan"])
+def test_direct_level_singular(n, kind):
+    """A level with a pivot of 0 (a row or column of zeros, two equal rows, a
+    singular block beside a regular one) or an entry that is not finite: the
+    solve breaks down as the oracle's does and x is left as it was."""
+    d = _swapping_system(n, n)
+    own = np.repeat(np.arange(n), np.diff(d["rowptr"]))
+    k, v = n // 2, d["values"]
+    if kind == "zero row":
+        v[own == k] = 0.0
+    elif kind == "zero column":
+        v[d["col"] == k] = 0.0
+    elif kind == "loose block":
+        v[(own == k) != (d["col"] == k)] = 0.0
+        v[(own == k) & (d["col"] == k)] = 0.0
+    elif kind == "twin rows":
+        v[:] = np.where(d["col"] == own, 1.0, 0.0)
+        for i in (k, k + 1):        # rows k and k + 1: 1 in columns k and k + 1
+            at = np.arange(d["rowptr"][i], d["rowptr"][i + 1])
+            v[at] = np.where((d["col"][at] == k) | (d["col"][at] == k + 1), 1.0, 0.0)
+    else:
+        v[d["rowptr"][k] + 1] = np.inf if kind == "inf" else np.nan
+    d["x0"] = np.full(n, 0.25)
+    g, o = gpu_solve(d), _oracle.OracleSolver().solve(d)
+    assert g[:2] == o[:2] and g[0] == 2 and np.isnan(g[2]) and np.isnan(o[2]), (g[:3], o[:3])
+    assert np.array_equal(g[3], d["x0"])

@@ -5,7 +5,8 @@
 // Step k of that algorithm swaps rows k and p_k (the pivot row), divides row
 // k by the pivot and subtracts f_k(i) times it from every other row i, f_k
 // being column k before the division.  Two facts make it cheaper without
-// changing an operation on a value that can differ from 0:
+// changing an operation on a value that can differ from 0 (a pivot that is 0
+// or not finite aside, see the end):
 //
 //  * In place.  Column n + o of [A | I] stays the unit vector of row o's
 //    present position until row o is taken as a pivot row (its entry in row
@@ -34,7 +35,12 @@
 //
 // A multiplier of 0 leaves the element as it is even where the row is not
 // finite; the wide update tests that only where a row of the step is not
-// finite (a singular level).
+// finite (a singular level).  On [A | I] a pivot of 0 makes 0 / 0 in row k of
+// the columns not yet taken, which are not held here.  Their slots' own row k
+// is divided by that 0 too, so row k ends without a finite entry, and so does
+// every row with a multiplier other than 0, in either form; the other rows are
+// not touched.  A place may hold an infinity here and a NaN there: a run's
+// first half step makes a NaN of both.
 #pragma once
 
 #include "yz_common.cuh"
@@ -192,7 +198,7 @@ __device__ __forceinline__ void GjApply(int n, double *__restrict__ Mc, const Gj
 }
 
 //  The panel of bN <= B slots from kN on, run through its steps: a thread
-//  holds R rows, t + 1024 r.  Records the pivots and the multipliers (the
+//  holds R rows, t + 512 r.  Records the pivots and the multipliers (the
 //  column of step c after its swap, n a step) and leaves the slots' columns
 //  of the inverse in Mc.
 template<int B, int R>
