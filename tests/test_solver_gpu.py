@@ -684,3 +684,39 @@ def test_direct_level_singular(n, kind):
     g, o = gpu_solve(d), _oracle.OracleSolver().solve(d)
     assert g[:2] == o[:2] and g[0] == 2 and np.isnan(g[2]) and np.isnan(o[2]), (g[:3], o[:3])
     assert np.array_equal(g[3], d["x0"])
+
+
+_SHAPE_CHILD = r"""
+import json, sys
+sys.path[:0] = [sys.argv[1], sys.argv[1] + "/tests", sys.argv[1] + "/tests/golden"]
+import numpy as np
+import _systems
+import yuzen_b200 as yz
+import test_solver_gpu as t
+d = _systems.film_system(int(sys.argv[2]), seed=11)
+out = []
+for shape in ((-1, 0, 0), (int(sys.argv[3]), 0, 0)):
+    be = yz.B200Backend()
+    be.SetPrecision(yz.PREC_FP32_CYCLE)
+    be.SetTuning(*shape)
+    be.SetGraphLoop(False)
+    g = t.gpu_solve(d, backend=be)
+    out.append([g[0], g[1], be.launches(), g[3].tobytes().hex()[:4096]])
+print(json.dumps(out))
+"""
+
+
+@pytest.mark.parametrize("N,fuse", [(100, 0), (384, 0), (384, 1)])
+def test_fuse_from_in_the_environment_is_a_launch_shape(N, fuse):
+    """YZ_FUSE_FROM asks for the separate launches as SetTuning does: the same
+    launches and bits, with no cluster in their place."""
+    import json
+    import os
+    import subprocess
+    import sys
+    root = Path(__file__).resolve().parents[1]
+    r = subprocess.run([sys.executable, "-c", _SHAPE_CHILD, str(root), str(N), str(fuse)], capture_output=True, text=True,
+                       env=dict(os.environ, YZ_FUSE_FROM=str(fuse)), timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
+    env, tuned = json.loads(r.stdout.strip().splitlines()[-1])
+    assert env[0] == 0 and env == tuned, (env[:3], tuned[:3])

@@ -916,19 +916,31 @@ void Solver::LaunchCoarseCycle()
 	CountLaunches(1);
 }
 
-//  YZ_FUSE_FROM: the first level (1 or more) of the FP32 cycle whose way down
-//  and way up each run as one launch; 0 switches the fused form off.  The
-//  default, 2, is the measured best on the 512^2 film (four levels of
-//  266,256 / ~30,000 / ~3,500 / ~400 rows): from level 1 the recomputation
-//  costs what the launches save (the same solve time with a quarter fewer
-//  launches), from level 2 the solve is 3 % faster than with no fusion.
-//  SetTuning overrides it for one context.
-int Solver::FusedFrom() const
+//  The first level (1 or more) of the FP32 cycle whose way down and way up
+//  each run as one launch.  The default, 2, was the best of the separate
+//  launches on the 512^2 film (four levels of 266,256 / ~30,000 / ~3,500 /
+//  ~400 rows): from level 1 the recomputation costs what the launches save
+//  (the same solve time with a quarter fewer launches), from level 2 the solve
+//  was 3 % faster than with no fusion.  Where the second coarse level has at
+//  most 8,000 rows (films up to about 1,180^2) the cluster takes it before the
+//  fused form is reached (LaunchCoarse).  YZ_FUSE_FROM (0: none) or SetTuning,
+//  for one context, override the default and keep the cluster away.
+static int FuseFromEnv()
 {
 	static const char *env = std::getenv("YZ_FUSE_FROM");
-	static const int k = env ? (std::atoi(env) > 0 ? std::atoi(env) : 1 << 30) : 2;
-	if(_fuseFrom == 0) return 1 << 30;
-	return _fuseFrom > 0 ? _fuseFrom : k;
+	static const int k = !env ? -1 : std::atoi(env) > 0 ? std::atoi(env) : 0;
+	return k;
+}
+
+int Solver::FusedFrom() const
+{
+	const int k = _fuseFrom >= 0 ? _fuseFrom : FuseFromEnv();
+	return k > 0 ? k : k == 0 ? 1 << 30 : 2;
+}
+
+bool Solver::ShapesSet() const
+{
+	return _precision != YZ_PREC_FP64 && (_fuseFrom >= 0 || _coarseLanes > 0 || FuseFromEnv() >= 0);
 }
 
 //  The FP32 cycle's post-smoothing at the finest level (the FP64 cycle keeps

@@ -133,9 +133,9 @@ private:
 	void ClearBounds();
 	void ProbeSweeps();
 	void EnqueueProbe();
-	//  launch shapes asked for (SetTuning) on the FP32 cycle's separate
-	//  launches: the one-cluster forms stand back
-	bool ShapesSet() const { return _precision != YZ_PREC_FP64 && (_fuseFrom >= 0 || _coarseLanes > 0); }
+	//  launch shapes asked for (SetTuning, YZ_FUSE_FROM) on the FP32 cycle's
+	//  separate launches: the one-cluster forms stand back
+	bool ShapesSet() const;
 	void CoarseDown(int lanes, int nc, const Level &L, const float *f, float *fc);
 	void CoarseUp(int lanes, const Level &L, const float *f, const float *xc, float *x);
 	const int *Halt() const { return &_sc.get()->state; }
