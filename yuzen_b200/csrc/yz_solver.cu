@@ -1382,9 +1382,10 @@ void Solver::RunIterations(int kind)
 	//  and buffers stay those it was captured with (the same pattern and
 	//  precision and, for the AMG kind, the same hierarchy: a reused one),
 	//  and captured anew otherwise (0.2-0.5 ms, less than the host launches
-	//  it saves on the 512^2 film).  YZ_GRAPH=0, the context's switch off
-	//  (SetGraphLoop), or a kernel being timed: the iterations are launched
-	//  from the stream instead.
+	//  it saves on the 512^2 film).  A small system's run is one cluster's
+	//  instead (ClusterRun).  YZ_GRAPH=0, a kernel being timed, or, where the
+	//  cluster does not take the run, the context's switch off (SetGraphLoop):
+	//  the iterations are launched from the stream.
 	static const char *env = std::getenv("YZ_GRAPH");
 	static const bool graphOff = env && env[0] == '0';
 	LoopGraph &lg = _loop[kind];
@@ -1401,7 +1402,9 @@ void Solver::RunIterations(int kind)
 		++hooks;
 	};
 	if(collect) _zs.reserve((size_t)_n);
-	if(graphOff || TimingActive() || collect || (!_graphLoop && (kind == kPrecLearned || _n > ClusterRows() || ShapesSet())))
+	const bool launched = graphOff || TimingActive() || collect;
+	const bool cluster = !launched && ClusterRun(kind);
+	if(launched || (!cluster && !_graphLoop))
 	{
 		//  one iteration kept in flight: the state after iteration k is
 		//  copied to pinned memory and read while iteration k+1 runs; the
@@ -1444,7 +1447,6 @@ void Solver::RunIterations(int kind)
 		if(collect) { --_collectLeft; _collected += hooks; }
 		return;
 	}
-	const bool cluster = ClusterRun(kind);
 	if(!cluster)
 	{
 		if(lg.exec == nullptr || lg.key != key)
