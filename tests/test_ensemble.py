@@ -36,6 +36,13 @@ def test_batch_is_seeded_and_in_range():
     assert len({c.Nx for c in cases.batch(256)}) == 5
 
 
+def test_autotune_candidates_differ():
+    """No shape is timed twice: 0 sweeps are the library's 8."""
+    from yuzen_b200 import autotune
+    shapes = [(f, lanes, sweeps or 8) for f, lanes, sweeps in autotune.CANDIDATES]
+    assert len(set(shapes)) == len(shapes) and shapes[0] == (-1, 0, 8)
+
+
 def test_autotune_classes_and_summary():
     from yuzen_b200 import PREC_FP64, autotune
     batch = cases.batch(32)

@@ -26,8 +26,9 @@ from . import step as ys
 
 #  (first fused level, lanes a row, finest-level sweeps): the library's
 #  default (-1, 0, 0), no fusion, fusion from level 1, fixed lane counts, and
-#  fewer and more sweeps
-CANDIDATES = ((-1, 0, 0), (0, 0, 0), (1, 0, 0), (-1, 4, 0), (-1, 8, 0), (0, 8, 0), (-1, 0, 3), (-1, 0, 8))
+#  fewer sweeps than the default's 8 (the most).  A fusion level or a lane
+#  count asks for the separate launches; the others keep the one-cluster forms
+CANDIDATES = ((-1, 0, 0), (0, 0, 0), (1, 0, 0), (-1, 4, 0), (-1, 8, 0), (0, 8, 0), (-1, 0, 3), (-1, 0, 5))
 
 
 def size_classes(cases) -> dict:
