@@ -717,6 +717,7 @@ __global__ void __launch_bounds__(kGemmThreads) KGemmWarp(int nx, const int *__r
 			const int c = tc[q + l];
 			const double v = tv[q + l];
 			const unsigned mask = __ballot_sync(all, c >= 0);
+			__syncwarp();		// a lane's place may be where another has just read
 			if(c >= 0) { const int to = at + __popc(mask & lt); tc[to] = c; tv[to] = v; }
 			at += __popc(mask & gm);
 			__syncwarp();
