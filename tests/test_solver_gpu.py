@@ -720,3 +720,24 @@ def test_fuse_from_in_the_environment_is_a_launch_shape(N, fuse):
     assert r.returncode == 0, r.stderr[-2000:]
     env, tuned = json.loads(r.stdout.strip().splitlines()[-1])
     assert env[0] == 0 and env == tuned, (env[:3], tuned[:3])
+
+
+@pytest.mark.parametrize("stiff,most", [(1.0, 10), (100.0, 64)])
+@pytest.mark.parametrize("N", [60, 160])
+def test_chebyshev_sweeps_pay_on_stiff_films(N, stiff, most):
+    """A smooth film (constant coefficients) in the FP32 cycle, inside one
+    cluster (60) and as separate launches (160): eight Chebyshev sweeps take
+    the iterations that a restatement of the cycle in float32 takes (7 and 7
+    at stiff 1, 45 and 49 at 100) within a third and one, which wrong bounds
+    or weights would not, and fewer than two thirds of one sweep's."""
+    d = _systems.upwind_system(N, 0.0, stiff)
+    assert _oracle.OracleSolver().solve(d)[0] == 0
+    its = []
+    for sweeps in (8, 1):
+        be = yz.B200Backend()
+        be.SetPrecision(yz.PREC_FP32_CYCLE)
+        be.SetTuning(-1, 0, sweeps)
+        g = gpu_solve(d, be)
+        assert g[0] == 0 and _true_residual(d, g[3]) <= 2e-10, g[:3]
+        its.append(g[1])
+    assert its[0] <= most and 3 * its[0] < 2 * its[1], its
