@@ -66,3 +66,16 @@ def test_struct_layouts_match_the_header(tmp_path):
         want.append(f"{cname} size {ctypes.sizeof(py)}")
         want += [f"{cname} {fname} {getattr(py, fname).offset}" for fname, _ in py._fields_]
     assert [g for g in got if g] == want
+
+
+def test_build_without_the_reference_sources(tmp_path, monkeypatch):
+    """An empty folder in the reference's place: the library and the oracle
+    are built, the binaries made from the reference's sources are left out."""
+    monkeypatch.syspath_prepend(str(HEADER.parents[1]))
+    monkeypatch.setenv("YZ_REFERENCE", str(tmp_path))
+    import __graft_entry__ as entry
+    ran = []
+    real = entry.subprocess.run
+    monkeypatch.setattr(entry.subprocess, "run", lambda cmd, **kw: ran.append(cmd) or real(cmd, **kw))
+    entry.build()
+    assert [c[-1] for c in ran if c[0] == "make"] == ["solver"]
