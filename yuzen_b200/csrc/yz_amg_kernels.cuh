@@ -876,9 +876,20 @@ __global__ void KPostSmooth(const int *__restrict__ halt, int n, const int *__re
 //  sweeps missed advection in 1 % of the area.
 //
 //  Both errors go side by side (x: Chebyshev, y: weight 1), so that 16 sweeps
-//  read the matrix 16 times and not 32.
+//  read the matrix 16 times and not 32: a 640^2 step of four set-ups took 75 us
+//  a set-up more with a row sum each, 17 with one of pairs.
 //--------------------------------------------------------------------------
-__global__ void KProbeStart(int n, float2 *__restrict__ x, double *lam)
+struct __align__(8) ProbePair
+{
+	float x, y;
+	ProbePair() = default;
+	__device__ __forceinline__ explicit ProbePair(float a) : x(a), y(a) {}
+	__device__ __forceinline__ ProbePair(float a, float b) : x(a), y(b) {}
+};
+__device__ __forceinline__ ProbePair operator*(ProbePair a, ProbePair b) { return ProbePair(a.x * b.x, a.y * b.y); }
+__device__ __forceinline__ ProbePair operator+(ProbePair a, ProbePair b) { return ProbePair(a.x + b.x, a.y + b.y); }
+
+__global__ void KProbeStart(int n, ProbePair *__restrict__ x, double *lam)
 {
 	if(blockIdx.x == 0 && threadIdx.x == 0) lam[2] = 0.0;
 	for(int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -888,35 +899,33 @@ __global__ void KProbeStart(int n, float2 *__restrict__ x, double *lam)
 		u = (u ^ (u >> 13)) * 3266489917u;
 		u ^= u >> 16;
 		const float v = (float)(int)(u >> 8) * (1.0f / 8388608.0f) - 1.0f;
-		x[i] = make_float2(v, v);
+		x[i] = ProbePair(v);
 	}
 }
 
 __global__ void KProbeSweep(int n, const int *__restrict__ ptr, const int *__restrict__ sellOff,
                             const __grid_constant__ Sten sn, const int *__restrict__ col, const float *__restrict__ val,
-                            const float *__restrict__ M, const float2 *__restrict__ x, float2 *__restrict__ xout,
+                            const float *__restrict__ M, const ProbePair *__restrict__ x, ProbePair *__restrict__ xout,
                             const double *__restrict__ lam, double ck, double ir)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if(i >= n) return;
 	const float w = (float)ChebWeight(lam, ck, ir);
-	const float sx = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return x[c].x; });
-	const float sy = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return x[c].y; });
-	const float2 xi = x[i];
+	const ProbePair s = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return x[c]; }), xi = x[i];
 	const float m = M[i];
-	xout[i] = make_float2(xi.x - w * m * sx, xi.y - m * sy);
+	xout[i] = ProbePair(xi.x - w * m * s.x, xi.y - m * s.y);
 }
 
 //  what is left of either; a sum that is not finite counts as more than one
 //  that is
-__global__ void __launch_bounds__(kRT) KProbeJudge(int n, const float2 *__restrict__ x, RedScratch rs, double *lam)
+__global__ void __launch_bounds__(kRT) KProbeJudge(int n, const ProbePair *__restrict__ x, RedScratch rs, double *lam)
 {
 	__shared__ double sh[2 * kRT];
 	double a[2] = {0.0, 0.0}, tot[2];
 	const int i = blockIdx.x * kRT + threadIdx.x;
 	if(i < n)
 	{
-		const float2 v = x[i];
+		const ProbePair v = x[i];
 		a[0] = (double)v.x * (double)v.x;
 		a[1] = (double)v.y * (double)v.y;
 	}

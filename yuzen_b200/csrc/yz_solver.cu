@@ -968,7 +968,9 @@ void Solver::ClearBounds()
 //  its own beside the rest of the set-up, which leaves most of the chip idle,
 //  and as one graph, for the host's time to queue 18 launches is the set-up's:
 //  a 301^2 set-up of 1.9 ms took 88 us more with them in line, 55 us more
-//  queued beside it, and 4 us more so.
+//  queued beside it, and 4 to 30 us more so.  A step of three set-ups, without
+//  and with the trial: 60^2 5.86 and 5.91 ms, 300^2 4.69 and 4.78, 640^2 13.38
+//  and 13.44.
 void Solver::ProbeSweeps()
 {
 	if(!_stProbe)
@@ -1015,7 +1017,7 @@ void Solver::EnqueueProbe()
 {
 	Level &L = *_levels[0];
 	const int n = L.n, K = FineSweeps();
-	float2 *x = reinterpret_cast<float2 *>(_ph.get()), *y = reinterpret_cast<float2 *>(_sh.get());
+	ProbePair *x = reinterpret_cast<ProbePair *>(_ph.get()), *y = reinterpret_cast<ProbePair *>(_sh.get());
 	YZ_LAUNCH(KProbeStart, GridFor(n, kB), kB, 0, _stProbe, n, x, _lam.get());
 	for(int k = 0; k < 2 * K; ++k)
 	{
