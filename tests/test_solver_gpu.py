@@ -405,7 +405,7 @@ def test_fused_coarse_levels_match_the_separate_kernels(precision):
 def test_tuning_shapes_and_sweeps():
     """yz_solver_set_tuning: out-of-range shapes are usage errors; every shape
     solves the 384^2 film to the tolerance in the FP32 cycle, and the finest
-    level's five default sweeps take fewer iterations than the reference's
+    level's eight default sweeps take fewer iterations than the reference's
     one."""
     d = _systems.film_system(384, seed=11)
     be = yz.B200Backend()
@@ -456,8 +456,8 @@ def _swapping_system(n: int, seed: int) -> dict:
 @pytest.mark.parametrize("n", [1, 2, 15, 17, 31, 33, 65, 255, 257, 511, 513, 1023, 1025, 1100])
 def test_direct_level_bitwise(n):
     """The direct level's inverse (yz_gj.cuh) around its widths: a column
-    tile (16), a panel (32 slots, fewer above ~810 rows), the rows a block
-    takes side by side (256, 512, 1024)."""
+    tile (16), a panel (16 slots, 8 above 1,024 rows), the rows a block takes
+    side by side (512, twice that with two rows a thread)."""
     d = _swapping_system(n, n)
     assert_same(gpu_solve(d)[:4], _oracle.OracleSolver().solve(d))
 

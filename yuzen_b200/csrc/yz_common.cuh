@@ -212,7 +212,8 @@ __device__ __forceinline__ double LaneTree(const double *v, int t)
 	return s;
 }
 
-//  Fold Q values per thread over a block of 256 (same order as Tree256).
+//  Fold Q values per thread over a block of 256 (same order as the
+//  oracle's Tree256).
 //  sh: Q*256 doubles of shared memory.  Result valid in thread 0.
 template<int Q>
 __device__ __forceinline__ void BlockTree(double (&a)[Q], double *sh)
