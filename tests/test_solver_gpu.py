@@ -741,3 +741,22 @@ def test_chebyshev_sweeps_pay_on_stiff_films(N, stiff, most):
         assert g[0] == 0 and _true_residual(d, g[3]) <= 2e-10, g[:3]
         its.append(g[1])
     assert its[0] <= most and 3 * its[0] < 2 * its[1], its
+
+
+def test_set_up_without_an_iteration_is_no_yardstick():
+    """A hierarchy set up at a solve that needed no iteration (the guess was
+    the answer) is held to the next solve's count: it serves on."""
+    d = dict(_systems.film_system(100, seed=4), epsilon=1e-10)
+    pat = yz.CrsPattern(d["rowptr"], d["col"], d["sorted_col"], d["sorted_src"])
+    s = yz.LinearSolverSettings(2, True, 500, 1e-10, False)
+    x = np.zeros(d["n"])
+    assert yz.B200Backend().Solve(yz.LinearSolverSettings(2, True, 500, 1e-12, False), pat, d["values"], d["rhs"], x)[0] == 0
+    be = yz.B200Backend()
+    be.SetAmgReuse(64)
+    ran = []
+    for guess in (x, np.zeros(d["n"]), np.zeros(d["n"]), np.zeros(d["n"])):
+        l0 = be.launches()
+        it = be.Solve(s, pat, d["values"], d["rhs"], guess.copy())[1]
+        ran.append((it, be.launches() - l0))
+    assert ran[0][0] == 0 and ran[1][0] > 8, ran
+    assert ran[1] == ran[2] == ran[3] and ran[1][1] < ran[0][1], ran

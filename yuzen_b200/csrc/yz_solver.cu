@@ -1769,6 +1769,13 @@ int Solver::Solve(const yz_settings &set, const double *dValues, const double *d
 				//  iterations, 0.42 to 0.61 a digit; over nine films the count
 				//  varies by a factor of 5, the iterations a digit by 2.6 where
 				//  the set-up's solve took one, by 2.1 at most where it took more.)
+				//  (A set-up whose own solve took no iteration says nothing: the
+				//  next one that takes some stands for it.)
+				if(_freshIters == 0 && _sinceBuild < kYoungSolves)
+				{
+					_freshIters = it;
+					_freshRate = it / Digits(*_hsc);
+				}
 				if(it > _freshIters + std::max(4, _freshIters / 2))
 				{
 					if(_sinceBuild < kYoungSolves && it <= 4 + 2.0 * _freshRate * Digits(*_hsc)) _freshIters = it;
