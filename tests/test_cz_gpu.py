@@ -151,3 +151,21 @@ def test_learned_film_solves_meet_the_bar():
     assert st["learned_solves"] + st["learned_fallbacks"] >= 1, st
     print("learned film solves:", {k: st[k] for k in st if k.startswith("learned")},
           "film iterations", st["linear_iterations"], "reference", d["linear_iterations"])
+
+
+def test_fp32_cycle_keeps_the_large_films_iterations():
+    """The 256^2 x 16 film's solves take some 300 iterations, so the rounding
+    of the FP32 cycle's sweeps shows in their number: over 12 steps, with a
+    kept hierarchy, they take at most a quarter more than the FP64 cycle's
+    (sums of 12 steps scatter by about a tenth)."""
+    import yuzen_b200 as yz
+    from yuzen_b200 import cases
+    r = cases.cz_bumps(256, 16).record()
+    total = {}
+    for precision, reuse in ((yz.PREC_FP64, 0), (yz.PREC_FP32_CYCLE, 64)):
+        m = model(r)
+        m.set_precision(precision)
+        m.set_amg_reuse(reuse)
+        total[precision] = m.advance(12)["linear_iterations"]
+        m.close()
+    assert total[yz.PREC_FP32_CYCLE] <= 1.25 * total[yz.PREC_FP64], total

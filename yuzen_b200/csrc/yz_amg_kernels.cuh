@@ -842,23 +842,69 @@ __global__ void KProlong(const int *__restrict__ halt, int n, const int *__restr
 	}
 }
 
-//  xout = x + w m .* (f - A x); w 1, or (W) a step of the Chebyshev
-//  iteration on the bounds KSpai0 left
-template<class T, class TF, class TX, bool W = false>
+//  xout = x + m .* (f - A x)
+template<class T, class TF, class TX>
 __global__ void KPostSmooth(const int *__restrict__ halt, int n, const int *__restrict__ ptr,
                             const int *__restrict__ sellOff, const __grid_constant__ Sten sn, const int *__restrict__ col,
                             const T *__restrict__ val, const T *__restrict__ M, const TF *__restrict__ f,
-                            const T *__restrict__ x, TX *__restrict__ xout, const double *__restrict__ lam, double ck, double ir)
+                            const T *__restrict__ x, TX *__restrict__ xout)
 {
 	PdlEntry();
 	if(halt && *halt) return;
-	const T w = W ? (T)ChebWeight(lam, ck, ir) : T(1);
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	if(i < n)
 	{
 		const T fi = (T)f[i], xi = x[i], mi = M[i];
 		const T s = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return x[c]; });
-		xout[i] = (TX)(xi + (W ? w * mi : mi) * (fi - s));
+		xout[i] = (TX)(xi + mi * (fi - s));
+	}
+}
+
+//  The finest level's sweeps of the FP32 cycle, on the correction: the
+//  residual r = f - A x once, then e = w m r (KSweepFirst), e = e + w m (r -
+//  A e) (KSweepNext), and x + e at the last (KSweepLast); w a step of the
+//  Chebyshev iteration on the bounds KSpai0 left, or 1 (ChebWeight).  On x
+//  itself every sweep rounds A x, which is small against x's smooth part, and
+//  a step's weight is up to 9 times a plain sweep's.  (BiCGStab iterations a
+//  step of the 256^2 ConcZ film, the same order of the weights: 715 and 716 on
+//  x, 650 and 641 so; Solver::SweepRoot has the order's part.)
+template<class T, class TF>
+__global__ void KSweepFirst(const int *__restrict__ halt, int n, const int *__restrict__ ptr,
+                            const int *__restrict__ sellOff, const __grid_constant__ Sten sn, const int *__restrict__ col,
+                            const T *__restrict__ val, const T *__restrict__ M, const TF *__restrict__ f,
+                            const T *__restrict__ x, T *__restrict__ r, T *__restrict__ e, const double *__restrict__ lam,
+                            double ck, double ir)
+{
+	PdlEntry();
+	if(halt && *halt) return;
+	const T w = (T)ChebWeight(lam, ck, ir);
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i < n)
+	{
+		const T fi = (T)f[i], mi = M[i];
+		const T ri = fi - RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return x[c]; });
+		r[i] = ri;
+		e[i] = w * mi * ri;
+	}
+}
+
+template<class T, class TX, bool Last>
+__global__ void KSweepNext(const int *__restrict__ halt, int n, const int *__restrict__ ptr,
+                           const int *__restrict__ sellOff, const __grid_constant__ Sten sn, const int *__restrict__ col,
+                           const T *__restrict__ val, const T *__restrict__ M, const T *__restrict__ r,
+                           const T *__restrict__ e, const T *__restrict__ x, TX *__restrict__ out, const double *__restrict__ lam,
+                           double ck, double ir)
+{
+	PdlEntry();
+	if(halt && *halt) return;
+	const T w = (T)ChebWeight(lam, ck, ir);
+	const int i = blockIdx.x * blockDim.x + threadIdx.x;
+	if(i < n)
+	{
+		const T ri = r[i], ei = e[i], mi = M[i], xi = Last ? x[i] : T(0);
+		const T s = RowSumSten(sn, i, ptr, sellOff, col, val, [&](int c) { return e[c]; });
+		const T en = ei + w * mi * (ri - s);
+		out[i] = (TX)(Last ? xi + en : en);
 	}
 }
 

@@ -365,26 +365,43 @@ __device__ __forceinline__ void ClCycle(const ClWho &who, const ClPlan<T> &P, co
 		YZ_CL_FINE(i, n) L.xt[i] = ClProlongRow<T, double>(L, i, r, xc);
 	}
 	ClBarrier();
-	T *xin = L.xt, *xo = L.x;
-	for(int k = 1; k < P.sweeps; ++k)
+	if(P.sweeps == 1)
 	{
-		const T wk = (T)ChebWeight(P.lam, P.root[k - 1], P.ratio);
 		YZ_CL_FINE(i, n)
 		{
-			const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return xin[c]; });
-			xo[i] = xin[i] + wk * __ldg(L.M + i) * ((T)r[i] - s);
+			const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return L.xt[c]; });
+			z[i] = (double)(L.xt[i] + __ldg(L.M + i) * ((T)r[i] - s));
 		}
 		ClBarrier();
-		T *u = xin; xin = xo; xo = u;
+		return;
 	}
-	const T w = P.sweeps > 1 ? (T)ChebWeight(P.lam, P.root[P.sweeps - 1], P.ratio) : T(1);
-	YZ_CL_FINE(i, n)
+	//  the sweeps on the correction (KSweepFirst, KSweepNext): the residual in
+	//  t, the correction in x and f by turns
+	T *e = L.x, *eo = L.f;
+	for(int k = 0; k < P.sweeps; ++k)
 	{
-		const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return xin[c]; });
-		const T m = __ldg(L.M + i);
-		z[i] = (double)(xin[i] + (P.sweeps > 1 ? w * m : m) * ((T)r[i] - s));
+		const T w = (T)ChebWeight(P.lam, P.root[k], P.ratio);
+		const T *in = k == 0 ? L.xt : e;
+		YZ_CL_FINE(i, n)
+		{
+			const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return in[c]; });
+			const T m = __ldg(L.M + i);
+			if(k == 0)
+			{
+				const T ri = (T)r[i] - s;
+				L.t[i] = ri;
+				e[i] = w * m * ri;
+			}
+			else
+			{
+				const T en = e[i] + w * m * (L.t[i] - s);
+				if(k + 1 < P.sweeps) eo[i] = en;
+				else z[i] = (double)(L.xt[i] + en);
+			}
+		}
+		ClBarrier();
+		if(k > 0) { T *u = e; e = eo; eo = u; }
 	}
-	ClBarrier();
 }
 
 template<class A> __device__ __forceinline__ void ClCopy(A &to, const A &from)

@@ -743,13 +743,13 @@ void Solver::Cycle(size_t l, const double *f, double *x)
 		}
 		YZ_LAUNCH(KProlong, g, kB, 0, _st, Halt(), n, L.pptr.get(), L.pcol.get(), L.pval.get(), C.x.get(), x, L.xt.get());
 		YZ_LAUNCH(KPostSmooth, RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
-		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x, nullptr, 0.0, 0.0);
+		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x);
 	}
 	else
 	{
 		YZ_LAUNCH(KPreSmooth, g, kB, 0, _st, Halt(), n, L.M.get(), f, L.xt.get());
 		YZ_LAUNCH(KPostSmooth, RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), l == 0 ? _sellOff.get() : nullptr, StenOf(l),
-		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x, nullptr, 0.0, 0.0);
+		          l == 0 ? _sellCol.get() : L.col.get(), l == 0 ? _sellVal.get() : L.val.get(), L.M.get(), f, L.xt.get(), x);
 	}
 }
 
@@ -778,7 +778,7 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 		          val, L.M32.get(), f, L.x32.get(), L.t32.get());
 		LaunchCoarseCycle();
 		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
-		          L.M32.get(), f, L.xt32.get(), x, nullptr, 0.0, 0.0);
+		          L.M32.get(), f, L.xt32.get(), x);
 		return;
 	}
 	if(l + 1 < _nlev)
@@ -821,30 +821,30 @@ void Solver::Cycle32(size_t l, const TF *f, TX *x)
 		}
 		if(la == 1)
 		{
-			//  the finest level's sweeps: the Chebyshev iteration, float to
-			//  float (x32 and xt32 in turn) but for the last
-			const float *xin = L.xt32.get();
+			//  the finest level's sweeps on the correction, in x32 and f32 by
+			//  turns (level 0's f is the caller's vector)
 			const int K = l == 0 ? FineSweeps() : 1;
-			for(int k = 0; k + 1 < K; ++k)
-			{
-				float *xo = (xin == L.xt32.get()) ? L.x32.get() : L.xt32.get();
-				YZ_LAUNCH_PDL((KPostSmooth<float, TF, float, true>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col,
-				              val, L.M32.get(), f, xin, xo, _lam.get(), SweepRoot(k, K), kSweepRatio);
-				xin = xo;
-			}
 			if(K > 1)
-				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX, true>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
-				              L.M32.get(), f, xin, x, _lam.get(), SweepRoot(K - 1, K), kSweepRatio);
+			{
+				float *e = L.x32.get(), *eo = L.f32.get();
+				YZ_LAUNCH_PDL((KSweepFirst<float, TF>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
+				              L.M32.get(), f, L.xt32.get(), L.t32.get(), e, _lam.get(), SweepRoot(0, K), kSweepRatio);
+				for(int k = 1; k + 1 < K; ++k, std::swap(e, eo))
+					YZ_LAUNCH_PDL((KSweepNext<float, float, false>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l),
+					              col, val, L.M32.get(), L.t32.get(), e, nullptr, eo, _lam.get(), SweepRoot(k, K), kSweepRatio);
+				YZ_LAUNCH_PDL((KSweepNext<float, TX, true>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
+				              L.M32.get(), L.t32.get(), e, L.xt32.get(), x, _lam.get(), SweepRoot(K - 1, K), kSweepRatio);
+			}
 			else
 				YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val,
-				              L.M32.get(), f, xin, x, nullptr, 0.0, 0.0);
+				              L.M32.get(), f, L.xt32.get(), x);
 		}
 	}
 	else
 	{
 		YZ_LAUNCH_PDL((KPreSmooth<float, TF, float>), g, kB, 0, _st, Halt(), n, L.M32.get(), f, L.xt32.get());
 		YZ_LAUNCH_PDL((KPostSmooth<float, TF, TX>), RowBlocks(n), kB, 0, _st, Halt(), n, L.ptr.get(), so, StenOf(l), col, val, L.M32.get(), f,
-		          L.xt32.get(), x, nullptr, 0.0, 0.0);
+		          L.xt32.get(), x);
 	}
 }
 
@@ -955,7 +955,22 @@ bool Solver::ShapesSet() const
 //  all-physics 25, 5.0 -> 10, 2.7; 301^2 38, 7.1 -> 17, 4.5; 1024^2 162, 86 ->
 //  124, 80; 224^2 levelling 13, 2.1 -> 9, 1.5.  Five Chebyshev sweeps: 15, 3.3;
 //  24, 5.0; 145, 76; 13, 2.0.  YZ_FINE_SWEEPS or SetTuning override the 8.
-double Solver::SweepRoot(int k, int K) { return std::cos(3.14159265358979323846 * (2 * k + 1) / (2.0 * K)); }
+//
+//  The order of the roots.  From the least root to the largest, eight sweeps
+//  multiply the upper end of the spectrum by 396 before they damp it, and from
+//  the largest to the least they multiply the rounding of the first sweeps by as
+//  much; in the orders below (of all orders of K, the one whose leading and
+//  trailing partial products stay least on [0, hi], for a ratio of 20) neither
+//  passes 3.4 from K = 5 on, 2.4 at 8.  On the 256^2 ConcZ film, whose solves
+//  take 300 iterations, BiCGStab iterations a step (mean of 15, a hierarchy a
+//  solve / kept): ascending on x 877 / 953, with 1,741 in one step, this order on
+//  the correction (KSweepFirst) 650 / 641; five plain sweeps on x 661 / 685.
+double Solver::SweepRoot(int k, int K)
+{
+	static const int order[9][8] = {{0}, {0}, {0, 1}, {1, 0, 2}, {1, 3, 0, 2}, {1, 4, 2, 0, 3}, {2, 4, 0, 5, 1, 3},
+	                                {3, 5, 0, 4, 1, 6, 2}, {3, 5, 1, 7, 0, 4, 2, 6}};
+	return std::cos(3.14159265358979323846 * (2 * order[K][k] + 1) / (2.0 * K));
+}
 
 void Solver::ClearBounds()
 {
