@@ -370,11 +370,12 @@ __global__ void KSpai0(int n, const int *__restrict__ ptr, const int *__restrict
 //  weight 1 (KProbeJudge).
 __device__ __forceinline__ double ChebWeight(const double *lam, double ck, double ir)
 {
-	if(lam[2] != 0.0) return 1.0;
-	const double hi = lam[0], lo0 = lam[1];
+	//  the three read at once: a sweep of a small level waits for them
+	const double hi = lam[0], lo0 = lam[1], plain = lam[2];
 	double lo = hi * ir;
 	if(lo0 > lo && lo0 < hi) lo = lo0;
-	return 1.0 / (0.5 * ((hi + lo) - (hi - lo) * ck));
+	const double w = 1.0 / (0.5 * ((hi + lo) - (hi - lo) * ck));
+	return plain != 0.0 ? 1.0 : w;
 }
 
 //  damped Jacobi as a preconditioner: m_i = 0.72 * (1 / a_ii)

@@ -52,7 +52,8 @@ template<class T>
 struct ClPlan
 {
 	int count, sweeps;                       // levels; the finest level's post-smoothing sweeps
-	double root[8], ratio;                   // and, for more than one, their Chebyshev roots (ChebWeight)
+	double root[8], ratio;                   // and, for more than one, their Chebyshev roots
+	double weight[8];                        // and weights, taken at the kernel's start (ChebWeight)
 	const double *lam;
 	const int *so;                           // the finest level's SELL-32 slices
 	Sten sn;
@@ -365,7 +366,7 @@ __device__ __forceinline__ void ClCycle(const ClWho &who, const ClPlan<T> &P, co
 		YZ_CL_FINE(i, n) L.xt[i] = ClProlongRow<T, double>(L, i, r, xc);
 	}
 	ClBarrier();
-	if(P.sweeps == 1)
+	if(std::is_same<T, double>::value || P.sweeps == 1)
 	{
 		YZ_CL_FINE(i, n)
 		{
@@ -378,30 +379,34 @@ __device__ __forceinline__ void ClCycle(const ClWho &who, const ClPlan<T> &P, co
 	//  the sweeps on the correction (KSweepFirst, KSweepNext): the residual in
 	//  t, the correction in x and f by turns
 	T *e = L.x, *eo = L.f;
-	for(int k = 0; k < P.sweeps; ++k)
 	{
-		const T w = (T)ChebWeight(P.lam, P.root[k], P.ratio);
-		const T *in = k == 0 ? L.xt : e;
+		const T w = (T)P.weight[0];
 		YZ_CL_FINE(i, n)
 		{
-			const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return in[c]; });
-			const T m = __ldg(L.M + i);
-			if(k == 0)
-			{
-				const T ri = (T)r[i] - s;
-				L.t[i] = ri;
-				e[i] = w * m * ri;
-			}
-			else
-			{
-				const T en = e[i] + w * m * (L.t[i] - s);
-				if(k + 1 < P.sweeps) eo[i] = en;
-				else z[i] = (double)(L.xt[i] + en);
-			}
+			const T ri = (T)r[i] - ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return L.xt[c]; });
+			L.t[i] = ri;
+			e[i] = w * __ldg(L.M + i) * ri;
 		}
 		ClBarrier();
-		if(k > 0) { T *u = e; e = eo; eo = u; }
 	}
+	for(int k = 1; k + 1 < P.sweeps; ++k)
+	{
+		const T w = (T)P.weight[k];
+		YZ_CL_FINE(i, n)
+		{
+			const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return e[c]; });
+			eo[i] = e[i] + w * __ldg(L.M + i) * (L.t[i] - s);
+		}
+		ClBarrier();
+		T *u = e; e = eo; eo = u;
+	}
+	const T w = (T)P.weight[P.sweeps - 1];
+	YZ_CL_FINE(i, n)
+	{
+		const T s = ClRowSumFine(P.sn, i, L.ptr, P.so, L.col, L.val, [&](int c) { return e[c]; });
+		z[i] = (double)(L.xt[i] + (e[i] + w * __ldg(L.M + i) * (L.t[i] - s)));
+	}
+	ClBarrier();
 }
 
 template<class A> __device__ __forceinline__ void ClCopy(A &to, const A &from)
@@ -450,6 +455,8 @@ __global__ void __launch_bounds__(kClT, 1) KLoopCluster(const __grid_constant__ 
 	__shared__ ClPlan<T> P;
 	ClCopy(S, S0);
 	ClCopy(P, P0);
+	__syncthreads();
+	if(P.sweeps > 1 && (int)threadIdx.x < P.sweeps) P.weight[threadIdx.x] = ChebWeight(P.lam, P.root[threadIdx.x], P.ratio);
 	__syncthreads();
 	const ClWho who = ClSelf();
 	const int n = S.n;
