@@ -367,7 +367,7 @@ __global__ void KSpai0(int n, const int *__restrict__ ptr, const int *__restrict
 
 //  The weight of a Chebyshev step on [max(lo, hi / r), hi]: ck the cosine of
 //  the step's root, ir = 1 / r.  lam[2] not 0: the hierarchy takes sweeps of
-//  weight 1 (KProbeJudge).
+//  weight 1 (KProbeChoose).
 __device__ __forceinline__ double ChebWeight(const double *lam, double ck, double ir)
 {
 	//  the three read at once: a sweep of a small level waits for them
@@ -968,7 +968,7 @@ __global__ void KProbeSweep(int n, const int *__restrict__ ptr, const int *__res
 //  square n / 3) are good whatever the others leave: on a well conditioned
 //  system both leave 1e-5, a hair's breadth apart, and a hierarchy kept from one
 //  onto a stiffer film then took 24 iterations with plain sweeps, 13 with these.
-__global__ void __launch_bounds__(kRT) KProbeJudge(int n, const ProbePair *__restrict__ x, RedScratch rs, double *lam)
+__global__ void __launch_bounds__(kRT) KProbeChoose(int n, const ProbePair *__restrict__ x, RedScratch rs, double *lam)
 {
 	__shared__ double sh[2 * kRT];
 	double a[2] = {0.0, 0.0}, tot[2];

@@ -1040,7 +1040,7 @@ void Solver::EnqueueProbe()
 		          _sellVal32.get(), L.M32.get(), x, y, _lam.get(), SweepRoot(k % K, K), kSweepRatio);
 		std::swap(x, y);
 	}
-	YZ_LAUNCH(KProbeJudge, RedBlocks(n), kRT, 0, _stProbe, n, x, Red(5), _lam.get());
+	YZ_LAUNCH(KProbeChoose, RedBlocks(n), kRT, 0, _stProbe, n, x, Red(5), _lam.get());
 }
 
 int Solver::FineSweeps() const

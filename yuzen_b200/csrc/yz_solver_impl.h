@@ -23,7 +23,7 @@ struct Scal
 	int it, maxIter;         // iterations done, the cap
 	int state;               // 0 running; see KState
 	int bodies;              // iterations queued and run (the graph's loop count)
-	int plain;               // the cycle's finest level takes sweeps of weight 1 (KProbeJudge)
+	int plain;               // the cycle's finest level takes sweeps of weight 1 (KProbeChoose)
 };
 
 //  the state word of a BiCGStab run on the device
@@ -191,7 +191,7 @@ private:
 	DBuf<unsigned> _counters;
 	DBuf<Scal> _sc;
 	//  the FP32 cycle's finest level: bounds of the spectrum of M A (KSpai0), and
-	//  not 0 where its sweeps have weight 1 (KProbeJudge)
+	//  not 0 where its sweeps have weight 1 (KProbeChoose)
 	DBuf<double> _lam;
 	Scal *_hsc = nullptr;
 	int *_hint = nullptr;      // pinned: totals and flags read back together
